@@ -9,7 +9,7 @@ struct sclbm_domain {
     sclbm_params p{};
     uint8_t *d_mask = nullptr;
     void *buf[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}; // [parity][comp], 9N each
-    int parity = 0;                                             // buf[parity] holds the state
+    int parity = 0; // buf[parity] holds the state; turns over with every step
     void *rho_tmp[2] = {nullptr, nullptr}; // density arrays of the two-pass variant
     double *staging = nullptr;             // N doubles, host<->device conversions
     double *partials = nullptr;            // per-CTA partial sums of the monitor
@@ -19,6 +19,7 @@ struct sclbm_domain {
     int tile_y = 0;   // rows per tile (0: default)
     int tx = 128;     // threads per CTA
     bool has_solid = true; // the mask has solid nodes
+    bool batched = false;  // a batch holds, or once held, the buffers' addresses
     size_t bytes = 0; // device bytes held
 };
 

@@ -268,31 +268,59 @@ __device__ __forceinline__ void push_one_raw(const Fused2Args<S, T> &a, const in
     }
 }
 
-// Collide the node n.nb[0] from its populations f[k][i] (registers or shared
-// memory) and the density stencil, then push the results: the reference
-// sequence of src/lbm.cpp:177-204 (repulsive force), :250-269 (equilibrium
-// velocity), src/fluid.cpp:254-276 + src/lbm.cpp:305-311 (equilibrium, BGK),
-// :333-337 (volume force), :404-427 (stream with half-way bounce-back).
-template <typename S, typename T, int FLAGS, bool WIDE = false, typename Pops>
-__device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Pops &f,
-                                             const Stencil<T> &st, const Nbr &n)
-{
-    constexpr bool EXACT = sizeof(T) == 8;
-    constexpr bool FORCE = (FLAGS & KF_FORCE) != 0, SOLID = (FLAGS & KF_SOLID) != 0;
-    constexpr bool UNIFORM = SOLID && (FLAGS & KF_UNIFORM) != 0;
-    const uint32_t node = n.nb[0];
-    // a solid lane of the uniform form treats every neighbour as solid: its
-    // nine stores then land in its own slots, and carry zeros
-    const bool self_fluid = !SOLID || st.m[1][st.c] != 0;
-    if (SOLID && !UNIFORM && !self_fluid) {
-        // solid node: the reference's stream leaves zeros (src/lbm.cpp:431-434);
-        // on the domain path both buffers already hold them
+// Where a collided node's populations go.  A sink takes one component's
+// population (put), both components' populations of one direction (pair, in
+// the compute type; pair_half, already rounded to half storage), and the zeros
+// of a solid node (solid); node() is the lattice index of the node.
+// This one pushes into the output arrays of the launch.
+template <typename S, typename T, bool SOLID, bool WIDE> struct GlobalSink {
+    const Fused2Args<S, T> &a;
+    const Nbr &n;
+    __device__ __forceinline__ uint32_t node() const { return n.nb[0]; }
+    __device__ __forceinline__ void put(int k, int i, T v, uint32_t nf) const
+    {
+        push_one<S, T, SOLID, WIDE>(a, k, i, v, nf, n);
+    }
+    __device__ __forceinline__ void pair(int i, T v0, T v1, uint32_t nf) const
+    {
+        push_one<S, T, SOLID, WIDE>(a, 0, i, v0, nf, n);
+        push_one<S, T, SOLID, WIDE>(a, 1, i, v1, nf, n);
+    }
+    __device__ __forceinline__ void pair_half(int i, __half h0, __half h1, uint32_t nf) const
+    {
+        push_one_raw<S, SOLID, WIDE>(a, 0, i, h0, nf, n);
+        push_one_raw<S, SOLID, WIDE>(a, 1, i, h1, nf, n);
+    }
+    // the reference's stream leaves zeros at solid nodes (src/lbm.cpp:431-434);
+    // on the domain path both buffers already hold them
+    __device__ __forceinline__ void solid() const
+    {
         if (!a.solids_zero) {
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int i = 0; i < 9; ++i) Store<S>::st(a.fout[k] + elem<WIDE>(i, a.N, node), T(0));
+                for (int i = 0; i < 9; ++i) Store<S>::st(a.fout[k] + elem<WIDE>(i, a.N, n.nb[0]), T(0));
         }
+    }
+};
+
+// Collide one node from its populations f[k][i] (registers or shared memory)
+// and the density stencil, and hand the results to the sink: the reference
+// sequence of src/lbm.cpp:177-204 (repulsive force), :250-269 (equilibrium
+// velocity), src/fluid.cpp:254-276 + src/lbm.cpp:305-311 (equilibrium, BGK),
+// :333-337 (volume force), :404-427 (stream with half-way bounce-back).
+template <typename S, typename T, int FLAGS, typename Pops, typename Sink>
+__device__ __forceinline__ void collide_node(const Fused2Args<S, T> &a, const Pops &f,
+                                             const Stencil<T> &st, const Sink &sink)
+{
+    constexpr bool EXACT = sizeof(T) == 8;
+    constexpr bool FORCE = (FLAGS & KF_FORCE) != 0, SOLID = (FLAGS & KF_SOLID) != 0;
+    constexpr bool UNIFORM = SOLID && (FLAGS & KF_UNIFORM) != 0;
+    // a solid lane of the uniform form treats every neighbour as solid: its
+    // nine stores then land in its own slots, and carry zeros
+    const bool self_fluid = !SOLID || st.m[1][st.c] != 0;
+    if (SOLID && !UNIFORM && !self_fluid) {
+        sink.solid();
         return;
     }
     // nf[i] = 1 when the neighbour along c_i is a fluid node (mask bytes are 0 or 1)
@@ -353,15 +381,15 @@ __device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Po
                     fsx = a.c[k].gs_neg * Sx;
                     fsy = a.c[k].gs_neg * Sy;
                 } else {
-                    fsx = a.fsx[k][node];
-                    fsy = a.fsy[k][node];
+                    fsx = a.fsx[k][sink.node()];
+                    fsy = a.fsy[k][sink.node()];
                 }
                 const double io = a.c[k].inv_omega;
                 ux = ucx + Fx[k] * io / psi[k] + fsx * io;
                 uy = ucy + Fy[k] * io / psi[k] + fsy * io;
             } else {
-                ux = a.uex_old[k] ? a.uex_old[k][node] : 0.0;
-                uy = a.uey_old[k] ? a.uey_old[k][node] : 0.0;
+                ux = a.uex_old[k] ? a.uex_old[k][sink.node()] : 0.0;
+                uy = a.uey_old[k] ? a.uey_old[k][sink.node()] : 0.0;
             }
             double fe[9];
             feq_exact(psi[k], ux, uy, fe);
@@ -373,7 +401,7 @@ __device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Po
                     if (a.c[k].force_on) v += a.c[k].force[i];
                 }
                 if constexpr (UNIFORM) v = self_fluid ? v : 0.0;
-                push_one<S, T, SOLID, WIDE>(a, k, i, v, nf[i], n);
+                sink.put(k, i, v, nf[i]);
             }
         }
     } else {
@@ -458,8 +486,7 @@ __device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Po
                     h0 = self_fluid ? h0 : __float2half_rn(0.f);
                     h1 = self_fluid ? h1 : __float2half_rn(0.f);
                 }
-                push_one_raw<S, SOLID, WIDE>(a, 0, i, h0, nf[i], n);
-                push_one_raw<S, SOLID, WIDE>(a, 1, i, h1, nf[i], n);
+                sink.pair_half(i, h0, h1, nf[i]);
                 return sub2(fp(i), __half22float2(H));
             } else {
                 float v0 = V.x, v1 = V.y;
@@ -467,8 +494,7 @@ __device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Po
                     v0 = self_fluid ? v0 : 0.f;
                     v1 = self_fluid ? v1 : 0.f;
                 }
-                push_one<S, T, SOLID, WIDE>(a, 0, i, v0, nf[i], n);
-                push_one<S, T, SOLID, WIDE>(a, 1, i, v1, nf[i], n);
+                sink.pair(i, v0, v1, nf[i]);
                 return sub2(fp(i), V);
             }
         };
@@ -495,17 +521,24 @@ __device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Po
                 h0 = self_fluid ? h0 : __float2half_rn(0.f);
                 h1 = self_fluid ? h1 : __float2half_rn(0.f);
             }
-            push_one_raw<S, SOLID, WIDE>(a, 0, 0, h0, nf[0], n);
-            push_one_raw<S, SOLID, WIDE>(a, 1, 0, h1, nf[0], n);
+            sink.pair_half(0, h0, h1, nf[0]);
         } else {
             if constexpr (UNIFORM) {
                 V0.x = self_fluid ? V0.x : 0.f;
                 V0.y = self_fluid ? V0.y : 0.f;
             }
-            push_one<S, T, SOLID, WIDE>(a, 0, 0, V0.x, nf[0], n);
-            push_one<S, T, SOLID, WIDE>(a, 1, 0, V0.y, nf[0], n);
+            sink.pair(0, V0.x, V0.y, nf[0]);
         }
     }
+}
+
+// collide_node pushing into the launch's output arrays (n: the node and its
+// neighbours)
+template <typename S, typename T, int FLAGS, bool WIDE = false, typename Pops>
+__device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Pops &f,
+                                             const Stencil<T> &st, const Nbr &n)
+{
+    collide_node<S, T, FLAGS>(a, f, st, GlobalSink<S, T, (FLAGS & KF_SOLID) != 0, WIDE>{a, n});
 }
 
 // shared-memory view of one node's populations in a ring: f[k][i]

@@ -1,0 +1,318 @@
+// fused_two.cuh -- two time steps of a two-component FP32- or FP16-shifted
+// lattice in one launch.
+//
+// Why.  A step on its own reads and writes every population once, and the
+// one-step kernels run at the memory's copy rate on large lattices.  Two steps
+// per pass read and write the populations once for both: the state between the
+// steps lives in shared memory, a few rows at a time.  What bounds it then is
+// the FP32 pipe (packed instructions: 58 % busy) and, over seconds, the
+// board's power limit; DRAM is half busy.  Measured on one B200, us per step
+// (the one-step ring kernel before): FP32 4096^2 270 (407), its 60 % fluid
+// form 337 (459), FP16 4096^2 277 (334), FP32 1024^2 22.6 (35.5), 256^2 5.4
+// (8.2).  FP64 stays with the one-step kernels: its rows between the steps
+// leave two CTAs per SM, and 12 % busy warps ran no faster (398 against 388
+// on 4096 x 2048, 546 against 485 with solid nodes).
+//
+// Work decomposition.  A CTA of TX threads owns a strip of up to TX - 6
+// columns and a band of rows; thread t stands for column xb - 3 + t and
+// marches along the band.  One step reads densities one node around a node and
+// pushes one node further, so the second step's nodes need the first step's
+// results two nodes around them and the first densities three: the outer
+// three columns and rows are recomputed by neighbouring CTAs (same inputs,
+// same arithmetic, so the same values).  Iteration q of the march:
+//
+//   A  row q-3's densities after the first step, from the shared rows; row
+//      q's densities from its populations (registers, loaded during the
+//      previous iteration);                                       -- barrier
+//   B  collide row q-1 (first step), pushing into the shared rows q-2..q;
+//      request the populations of row q+1; collide row q-4 (second step),
+//      pushing into the output arrays;                            -- barrier
+//
+// Plain loads of one row ahead are enough here (half the bytes per step, and
+// a whole collision between request and use), so rows may start anywhere:
+// unlike the ring kernel this one has no alignment rule.
+//
+// The arithmetic per node is collide_node's, and the values between the steps
+// are held in the storage type, so the result equals two one-step launches
+// byte for byte.
+#pragma once
+#include "fused_step.cuh"
+
+namespace sclbm {
+
+// 128 threads: 256 ran 2-8 % slower (barrier over eight warps), 64 3-4 %
+// (halo columns)
+constexpr int TWO_TX = 128;
+
+// one direction of both components' populations between the steps
+template <typename S> struct TwoCell;
+template <> struct TwoCell<float> {
+    using type = float2;
+};
+template <> struct TwoCell<__half> {
+    using type = __half2;
+};
+
+// The rows between the steps, kept per direction only as long as they are
+// needed.  With the march pointing "ahead", the populations of row r that came
+// from behind (their direction points ahead) are pushed when row r-1 is
+// collided, the level ones with row r, and those that come back with row r+1,
+// half-way bounce-backs with row r; all are read two rows later.  Rings of
+// three, two and two rows of three directions each hold them.  Every slot has
+// one writer; slots of columns and rows that only feed the halo are never
+// read, and a solid node's slots never matter: densities and stencils are
+// masked.  28.7 KB for FP32: 113 KB of an SM stay with its L1 beside four CTAs.
+template <typename S, int TX> struct __align__(16) TwoShared {
+    static constexpr int ROW = 3 * TX; // three directions of a row
+    static constexpr int LEVEL = 3 * ROW, BEHIND = 5 * ROW;
+    typename TwoCell<S>::type m[7 * ROW];
+    float2 rho1[3][TX], rho2[3][TX]; // densities before the first and second step
+    uint8_t msk[8][TX];              // mask rows q-7 .. q
+};
+
+// place of direction i among the three of its class (opposite ones alike)
+__host__ __device__ constexpr int two_place(int i)
+{
+    return i == 0 || i == 2 || i == 4 ? 0 : (i == 1 || i == 5 || i == 7 ? 1 : 2);
+}
+
+// Offsets (elements of the row storage, this thread's column) of one row's
+// three classes of directions: c_y = -1, 0, +1.
+struct TwoRow {
+    int dn, level, up;
+    __device__ __forceinline__ int at(int i) const { return cy(i) == 0 ? level : (cy(i) > 0 ? up : dn); }
+};
+
+// pushes a first-step node's populations into the rows between the steps;
+// to: the destination rows of the three classes, own: the node's own row
+template <typename S, int TX, bool SOLID> struct SharedSink {
+    typename TwoCell<S>::type *m;
+    TwoRow to, own;
+    __device__ __forceinline__ int slot(int i, uint32_t nf) const
+    {
+        const int fwd = to.at(i) + two_place(i) * TX + cx(i);
+        if (i == 0 || !SOLID) return fwd;
+        const int back = own.at(opp(i)) + two_place(opp(i)) * TX;
+        return back ^ ((fwd ^ back) & (0 - (int)nf)); // nf is 0 or 1
+    }
+    __device__ __forceinline__ void pair(int i, float v0, float v1, uint32_t nf) const
+    {
+        m[slot(i, nf)] = make_float2(v0, v1);
+    }
+    __device__ __forceinline__ void pair_half(int i, __half h0, __half h1, uint32_t nf) const
+    {
+        m[slot(i, nf)] = __halves2half2(h0, h1);
+    }
+    __device__ __forceinline__ void solid() const {}
+};
+
+// populations of one row between the steps
+template <typename S, int TX>
+__device__ __forceinline__ void two_read(const TwoShared<S, TX> &sh, const TwoRow &r, float (&f)[2][9])
+{
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        float2 v;
+        if constexpr (sizeof(S) == 4) v = sh.m[r.at(i) + two_place(i) * TX];
+        else v = __half22float2(sh.m[r.at(i) + two_place(i) * TX]);
+        f[0][i] = v.x;
+        f[1][i] = v.y;
+    }
+}
+
+// wrap for offsets in [-3, n + 2] (n >= 3)
+__device__ __forceinline__ int wrap3(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
+
+// Two steps of the columns [xb, xb + ncol) and rows [y0, y0 + nrow) of a's
+// lattice (nx, ny >= 4), rows marched upward or (down) downward.
+template <typename S, int TX, int FLAGS>
+__device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const int xb, const int ncol,
+                                         const int y0, const int nrow, const bool down,
+                                         TwoShared<S, TX> &sh)
+{
+    using L = TwoShared<S, TX>;
+    constexpr bool SOLID = (FLAGS & KF_SOLID) != 0;
+    const int t = threadIdx.x;
+    const int nx = a.nx, ny = a.ny;
+    // columns of this thread that each stage computes
+    const bool load = t < ncol + 6;            // populations and densities before step 1
+    const bool step1 = t >= 1 && t < ncol + 5; // collisions of step 1
+    const bool dens2 = t >= 2 && t < ncol + 4; // densities before step 2
+    const bool step2 = t >= 3 && t < ncol + 3; // collisions of step 2
+    const int x = load ? wrap3(xb - 3 + t, nx) : 0;
+    const int xl = wrap1(x - 1, nx), xr = wrap1(x + 1, nx);
+    auto gy = [&](int q) { return wrap3(y0 + (down ? nrow - 1 - q : q), ny); };
+
+    uint8_t mask_ahead = 1;
+    // all-fluid lattices load on every thread (idle ones column 0): without the
+    // branch the loads of FP16 rows sit earlier (4096^2: 309 -> 289 us a step,
+    // FP32 286 -> 280); with solid nodes the branch was the faster form (337
+    // against 349)
+    auto load_row = [&](int q, float(&f)[2][9]) {
+        if (SOLID && !load) return;
+        const uint32_t node = (uint32_t)gy(q) * (uint32_t)nx + (uint32_t)x;
+        if (SOLID) mask_ahead = a.mask[node];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int i = 0; i < 9; ++i) f[k][i] = Store<S>::ld(a.fin[k] + elem<false>(i, a.N, node));
+    };
+    // all-fluid lattices ask L2 for the row after the one being loaded, one
+    // 128-byte line per thread (FP16 289 -> 277 us a step, FP32 1-2 %; with
+    // solid nodes within noise)
+    constexpr int LINES = (TX * (int)sizeof(S) + 127) / 128 + 1; // lines a row segment touches
+    const S *pf = nullptr;
+    if (!SOLID && t < 18 * LINES) {
+        const int arr = t / LINES, l = t % LINES;
+        const int col = min(max(xb - 3, 0) + l * (128 / (int)sizeof(S)), nx - 1);
+        pf = a.fin[arr >= 9 ? 1 : 0] + (size_t)(arr % 9) * a.N + col;
+    }
+
+    // slots of the rows q (s0), q - 1 (s1), q - 2 (s2) of the rings of three;
+    // rows three apart share one
+    int s0 = 0, s1 = 2, s2 = 1;
+    // the classes of row r (any value of its parity) whose slot in the rings of
+    // three is s
+    auto row_at = [&](int s, int r) {
+        const int ahead = s * L::ROW + t, two = (r & 1) * L::ROW + t;
+        return TwoRow{down ? ahead : L::BEHIND + two, L::LEVEL + two, down ? L::BEHIND + two : ahead};
+    };
+    auto mrow = [&](int p) { return (const uint8_t *)sh.msk[(p + 8) & 7]; };
+
+    // cur: row q, prev: row q - 1, both before step 1; mcur: row q - 3, mprev:
+    // row q - 4, both after it
+    auto row = [&](const int q, float(&cur)[2][9], float(&prev)[2][9], float(&mcur)[2][9],
+                   const float(&mprev)[2][9]) {
+        if (dens2 && q >= 2 && q <= nrow + 3) {
+            float r0, r1;
+            two_read<S, TX>(sh, row_at(s0, q - 3), mcur);
+            node_density(mcur, r0, r1);
+            if (SOLID && !mrow(q - 3)[t]) r0 = r1 = 0.f;
+            sh.rho2[s0][t] = make_float2(r0, r1);
+        }
+        if (load && q <= nrow + 2) {
+            float r0, r1;
+            node_density(cur, r0, r1);
+            if (SOLID) {
+                if (!mask_ahead) r0 = r1 = 0.f;
+                sh.msk[(q + 8) & 7][t] = mask_ahead;
+            }
+            sh.rho1[s0][t] = make_float2(r0, r1);
+        }
+        __syncthreads();
+        const int lo = down ? s0 : s2, hi = down ? s2 : s0; // rows below and above the node
+        if (step1 && q >= -1 && q <= nrow + 2) {
+            const Stencil<float> st{{sh.rho1[lo], sh.rho1[s1], sh.rho1[hi]},
+                                    {mrow(down ? q : q - 2), mrow(q - 1), mrow(down ? q - 2 : q)}, t};
+            // ahead: row q; level: row q - 1; behind: row q - 2
+            const TwoRow own = row_at(s1, q - 1);
+            const int ahead = s0 * L::ROW + t, behind = L::BEHIND + (q & 1) * L::ROW + t;
+            const TwoRow to{down ? ahead : behind, own.level, down ? behind : ahead};
+            collide_node<S, float, FLAGS>(a, prev, st, SharedSink<S, TX, SOLID>{sh.m, to, own});
+        }
+        if (!SOLID) load_row(min(q + 1, nrow + 2), prev);
+        else if (q < nrow + 2) load_row(q + 1, prev);
+        if (!SOLID && pf != nullptr && q + 2 <= nrow + 2)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + (size_t)gy(q + 2) * (size_t)nx));
+        if (step2 && q >= 4 && q <= nrow + 3) {
+            const Stencil<float> st{{sh.rho2[lo], sh.rho2[s1], sh.rho2[hi]},
+                                    {mrow(down ? q - 3 : q - 5), mrow(q - 4), mrow(down ? q - 5 : q - 3)}, t};
+            const int yc = gy(q - 4);
+            const Nbr n = make_nbr(nx, x, xl, xr, yc, wrap1(yc - 1, ny), wrap1(yc + 1, ny));
+            collide_push<S, float, FLAGS>(a, mprev, st, n);
+        }
+        __syncthreads();
+        const int s = s2;
+        s2 = s1;
+        s1 = s0;
+        s0 = s;
+    };
+
+    float A[2][9], B[2][9], C[2][9], D[2][9];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 9; ++i) A[k][i] = B[k][i] = C[k][i] = D[k][i] = 0.f;
+    load_row(-3, A);
+    // two rows per trip so the register buffers swap roles instead of being copied
+    for (int q = -3; q <= nrow + 3; q += 2) {
+        row(q, A, B, C, D);
+        row(q + 1, B, A, D, C);
+    }
+}
+
+// Four CTAs per SM (128 registers, no spills).  A fifth needs 96 registers:
+// the spills and the smaller L1 beside five CTAs' shared memory cost a quarter
+// (362 against 288 us on 4096^2).
+constexpr int TWO_CTAS = 4;
+
+// strip s covers the columns [s*w, min(nx, (s+1)*w)), band b the rows
+// [b*ny/bands, (b+1)*ny/bands); neighbouring bands march in opposite
+// directions, so the rows they share are read by both near the same time
+template <typename S, int TX, int FLAGS>
+__global__ void __launch_bounds__(TX, TWO_CTAS)
+    k_two2(const __grid_constant__ Fused2Args<S, float> a, int w, int bands)
+{
+    __shared__ TwoShared<S, TX> sh;
+    const int band = blockIdx.y, xb = blockIdx.x * w;
+    const int y0 = (int)((long long)band * a.ny / bands);
+    const int nrow = (int)((long long)(band + 1) * a.ny / bands) - y0;
+    two_unit<S, TX, FLAGS>(a, xb, min(w, a.nx - xb), y0, nrow, (band & 1) != 0, sh);
+}
+
+// Strips of one width, as few as hold the lattice.
+inline int two_strips(int nx) { return (nx + TWO_TX - 7) / (TWO_TX - 6); }
+
+// Rows per band.  A band of r rows takes r + 8 iterations (six halo rows, two
+// to fill the pipeline).  With n CTAs on an SM an iteration takes as long as
+// the larger of its latency and n times a CTA's share of the SM; measured in
+// shares (0.48 us for FP32) the latency is about 1.8 of them, and four CTAs
+// are resident.  The rows with the least time over full waves and the last,
+// partial one are taken: 1024^2 16 rows (45 us a launch; 12 rows 55, 24 rows
+// 49), 256^2 3 rows (10.4; 6 rows 12.3), 4096^2 48 to 96 rows (within 2 %; 16
+// rows 8 % slower).
+inline int two_rows(int nx, int ny, int sms)
+{
+    const int cand[] = {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 56, 64};
+    int best = 2;
+    double least = 0.0;
+    for (int r : cand) {
+        const long units = (long)two_strips(nx) * ((ny + r - 1) / r), wave = (long)TWO_CTAS * sms;
+        const long rest = units % wave;
+        const double last = rest ? std::max(1.8, (double)((rest + sms - 1) / sms)) : 0.0;
+        const double cost = (r + 8) * ((double)(units / wave) * TWO_CTAS + last);
+        if (least == 0.0 || cost < least) {
+            least = cost;
+            best = r;
+        }
+    }
+    return best;
+}
+
+template <typename S, int TX, int FLAGS>
+inline cudaError_t launch_two2_f(const Fused2Args<S, float> &a, int rows, cudaStream_t s)
+{
+    const int strips = two_strips(a.nx);
+    const int w = (a.nx + strips - 1) / strips;
+    const int bands = std::min((a.ny + rows - 1) / rows, 65535);
+    k_two2<S, TX, FLAGS><<<dim3(strips, bands), TX, 0, s>>>(a, w, bands);
+    return cudaGetLastError();
+}
+
+// rows: rows per band (0: two_rows); lattices with solid nodes run the uniform
+// solid form.  Refuses lattices that need 64-bit offsets and those that a halo
+// of three wraps around more than once.
+template <typename S>
+inline cudaError_t launch_two2_any(const Fused2Args<S, float> &a, int rows, cudaStream_t s)
+{
+    if (needs_wide_offsets(a.N) || a.nx < 4 || a.ny < 4) return cudaErrorInvalidValue;
+    if (rows < 1) rows = two_rows(a.nx, a.ny, sm_count());
+    switch (kernel_flags(a)) {
+    case 0: return launch_two2_f<S, TWO_TX, 0>(a, rows, s);
+    case KF_FORCE: return launch_two2_f<S, TWO_TX, KF_FORCE>(a, rows, s);
+    case KF_SOLID: return launch_two2_f<S, TWO_TX, KF_SOLID | KF_UNIFORM>(a, rows, s);
+    default: return launch_two2_f<S, TWO_TX, KF_FORCE | KF_SOLID | KF_UNIFORM>(a, rows, s);
+    }
+}
+
+} // namespace sclbm

@@ -199,6 +199,10 @@ int ring_maps_of(const Fused2Args<__half, float> &a, int width, RingMaps *m);
 int async_resident_fp64(); // CTAs of the batched kernel resident on the device
 int async_resident_f32();
 constexpr int ASYNC_STRIP = 128;
+// two steps in one launch (fused_two.cuh): fin holds the state, fout receives
+// the state two steps later; rows per band (0 default)
+cudaError_t launch_two2_f32(const Fused2Args<float, float> &a, int rows, cudaStream_t s);
+cudaError_t launch_two2_f16(const Fused2Args<__half, float> &a, int rows, cudaStream_t s);
 // density pass (kernel a): rho (or rho - rho_ref for shifted storage) per node,
 // 0 at solid nodes; both components in one launch
 cudaError_t launch_density_fp64(const uint8_t *mask, const double *f0, const double *f1,

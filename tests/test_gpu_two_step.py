@@ -1,0 +1,90 @@
+"""Steps run in pairs (two per launch) against the one-step register tile.
+
+The pair kernel's nodes run the same arithmetic as the one-step kernels' and
+hold the state between the steps in the storage type, so the populations are
+equal byte for byte: at widths around its strips (122 columns), with bands of
+one row and of uneven heights, on lattices that its halo wraps around, for odd
+and even step counts.  The parity a batch relies on, and a captured step call,
+behave as with one step per launch.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def make(sclbm, nx, ny, prec, porous, force, seed=5):
+    from sc_lbm_b200 import workloads as W
+    n = nx * ny
+    mask = (W.uniform(seed, n) < 0.75).astype(np.int32) if porous else np.ones(n, np.int32)
+    F = (W.force_vec(1e-4, "x"), W.force_vec(2e-4, "y")) if force else (None, None)
+    p = sclbm.make_params(ncomp=2, tau=(1.0, 0.9), g_fluid=(0.9, 0.9), g_solid=(-0.1, 0.1),
+                          rho_ref=(1.0, 1.2), force=F)
+    f = [W.populations((1 + 0.2 * k) * (1 + 0.1 * (2 * W.uniform(seed + k, n) - 1)), mask)
+         for k in range(2)]
+
+    def build(variant=0, rows=0):
+        d = sclbm.Domain(nx, ny, mask, p, prec)
+        d.set_kernel(variant, rows)
+        for k in range(2):
+            d.upload_f(k, f[k])
+        return d
+    return build
+
+
+def state(d):
+    return [d.download_f(k).tobytes() for k in range(2)]
+
+
+@pytest.mark.parametrize("prec_name", ["FP32_SHIFTED", "FP16_SHIFTED"])
+@pytest.mark.parametrize("nx,ny,rows", [(4, 4, 0), (5, 7, 1), (64, 33, 5), (121, 20, 0), (122, 9, 4),
+                                        (123, 40, 32), (245, 31, 0), (1021, 77, 7)])
+def test_pairs_match_single_steps(sclbm, prec_name, nx, ny, rows):
+    prec = getattr(sclbm, prec_name)
+    for porous in (False, True):
+        for force in (False, True):
+            build = make(sclbm, nx, ny, prec, porous, force)
+            for steps in (2, 5):
+                a, b = build(0, rows), build(2, 0)
+                a.step(steps)
+                b.step(steps)
+                assert state(a) == state(b), (porous, force, steps)
+
+
+def test_pairs_keep_a_domain_in_step_with_its_batch(sclbm):
+    """Two steps outside the batch leave it usable, one does not."""
+    build = [make(sclbm, nx, 48, sclbm.FP32_SHIFTED, True, False) for nx in (96, 60)]
+    doms, alone = [b() for b in build], [b(2) for b in build]
+    doms[0].step(2)  # before the batch takes the buffers' addresses
+    batch = sclbm.Batch(doms)
+    doms[1].step(6)
+    batch.step(3)
+    alone[0].step(5)
+    alone[1].step(9)
+    for d, a in zip(doms, alone):
+        assert state(d) == state(a)
+    doms[1].step(1)
+    with pytest.raises(RuntimeError):
+        batch.step(1)
+
+
+def test_captured_steps_replay(sclbm):
+    import torch
+    build = make(sclbm, 130, 50, sclbm.FP32_SHIFTED, False, True)
+    d, one = build(), build(2)
+    st = torch.cuda.Stream()
+    sclbm.synchronize()
+    sclbm.set_stream(st.cuda_stream)
+    try:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            d.step(6)
+        with torch.cuda.stream(st):
+            for _ in range(3):
+                g.replay()
+        st.synchronize()
+        one.step(18)
+        assert state(d) == state(one)
+    finally:
+        sclbm.synchronize()
+        sclbm.set_stream(None)
