@@ -20,12 +20,13 @@
 #include "batch_kernel.cuh"
 #include "fused_async.cuh"
 #include "fused_ring.cuh"
+#include "fused_two.cuh"
 #include "tuning.h"
 
 
 using namespace sclbm;
 
-static constexpr int GRAPH_STEPS = 20; // launches per captured graph (even: parity returns)
+static constexpr int GRAPH_STEPS = 20; // steps per captured graph (a multiple of 4: the parity returns)
 
 struct sclbm_batch {
     std::vector<sclbm_domain *> doms;
@@ -57,6 +58,11 @@ struct sclbm_batch {
     RingMaps *d_maps[2] = {nullptr, nullptr};
     unsigned *d_counters = nullptr;
     int nunits[2] = {0, 0}, ring_grid[2] = {0, 0};
+    // steps in pairs (variant 0 of FP32/FP16 batches): units of the two-step
+    // kernel; absent (0) when a domain is too small for it
+    TwoUnit *d_two = nullptr;
+    int ntwo = 0;
+    bool use_two = false;
 };
 
 // the tile list of the current body
@@ -204,6 +210,72 @@ static int upload_args(sclbm_batch *b, const std::vector<int> &ty, const std::ve
     return build_rings<S, T>(b, h, ring_rows);
 }
 
+// Units of the two-step kernel: per domain its strips and bands, all of about
+// the rows that two_cost finds best for the batch's units (the caller's height
+// where given).  64 mixed domains: 24 rows 80 us per step, 16 rows 85, 32 rows
+// 98, 64 rows 92 (ring body 104).
+static int build_two(sclbm_batch *b, const int *tile_y)
+{
+    if (b->prec == SCLBM_FP64) return SCLBM_OK;
+    for (auto *d : b->doms)
+        if (d->nx < 4 || d->ny < 4) return SCLBM_OK;
+    auto bands_of = [&](const sclbm_domain *d, int k, int rows) {
+        const int r = tile_y && tile_y[k] > 0 ? tile_y[k] : rows;
+        return std::max(1, (int)((d->ny + r - 1) / r));
+    };
+    int rows = 1;
+    double least = 0.0;
+    for (int r : TWO_ROWS) {
+        long n = 0;
+        for (size_t k = 0; k < b->doms.size(); ++k) {
+            const int nx = (int)b->doms[k]->nx, w = two_width(nx);
+            n += (long)((nx + w - 1) / w) * bands_of(b->doms[k], (int)k, r);
+        }
+        const double cost = two_cost(n, r, sm_count());
+        if (least == 0.0 || cost < least) {
+            least = cost;
+            rows = r;
+        }
+    }
+    std::vector<TwoUnit> units;
+    std::vector<long> cost;
+    for (size_t k = 0; k < b->doms.size(); ++k) {
+        const sclbm_domain *d = b->doms[k];
+        const int w = two_width((int)d->nx), bands = bands_of(d, (int)k, rows);
+        for (int j = 0; j < bands; ++j) {
+            const int y0 = (int)((long long)d->ny * j / bands), y1 = (int)((long long)d->ny * (j + 1) / bands);
+            for (int xb = 0; xb < (int)d->nx; xb += w) {
+                units.push_back(TwoUnit{(int)k, xb, std::min(w, (int)d->nx - xb), y0, y1 - y0, j & 1});
+                cost.push_back(y1 - y0);
+            }
+        }
+    }
+    // largest first at domain granularity, as the ring's units
+    std::vector<long> dom_cost(b->doms.size(), 0);
+    for (size_t i = 0; i < units.size(); ++i)
+        dom_cost[units[i].dom] = std::max(dom_cost[units[i].dom], cost[i]);
+    std::vector<int> order(units.size());
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return dom_cost[units[x].dom] > dom_cost[units[y].dom]; });
+    std::vector<TwoUnit> sorted(units.size());
+    for (size_t i = 0; i < order.size(); ++i) sorted[i] = units[order[i]];
+    SCLBM_CUDA(cudaMalloc(&b->d_two, sorted.size() * sizeof(TwoUnit)));
+    SCLBM_CUDA(cudaMemcpy(b->d_two, sorted.data(), sorted.size() * sizeof(TwoUnit), cudaMemcpyHostToDevice));
+    b->ntwo = (int)sorted.size();
+    b->use_two = true;
+    return SCLBM_OK;
+}
+
+static cudaError_t batch_launch_two(sclbm_batch *b, int parity, cudaStream_t s)
+{
+    if (b->prec == SCLBM_FP32_SHIFTED)
+        return launch_batch_two_f32((const Fused2Args<float, float> *)b->d_args, b->d_two, b->ntwo, parity,
+                                    b->flags, s);
+    return launch_batch_two_f16((const Fused2Args<__half, float> *)b->d_args, b->d_two, b->ntwo, parity,
+                                b->flags, s);
+}
+
 extern "C" {
 
 void sclbm_batch_destroy(sclbm_batch *b)
@@ -221,6 +293,7 @@ void sclbm_batch_destroy(sclbm_batch *b)
         if (b->d_maps[r]) cudaFree(b->d_maps[r]);
     }
     if (b->d_counters) cudaFree(b->d_counters);
+    if (b->d_two) cudaFree(b->d_two);
     delete b;
 }
 
@@ -436,6 +509,7 @@ int sclbm_batch_create(sclbm_domain *const *domains, int ndomains, const int *ti
     if (!rc && cudaMemcpy(b->d_tiles_half, halves.data(), halves.size() * sizeof(TileRef),
                           cudaMemcpyHostToDevice) != cudaSuccess)
         rc = set_error(SCLBM_E_CUDA, "tile list upload");
+    if (!rc) rc = build_two(b, tile_y_per_domain);
     if (rc) {
         sclbm_batch_destroy(b);
         return rc;
@@ -468,6 +542,7 @@ int sclbm_batch_set_kernel(sclbm_batch *b, int variant)
               : variant == 10 ? BODY_WARP
               : variant == 0 ? b->auto_body
                              : BODY_TILE;
+    b->use_two = variant == 0 && b->ntwo > 0;
     for (auto &g : b->graph)
         if (g) {
             cudaGraphExecDestroy(g);
@@ -479,6 +554,11 @@ int sclbm_batch_set_kernel(sclbm_batch *b, int variant)
 int sclbm_batch_info(const sclbm_batch *b, int *ntiles, int *grid_ctas)
 {
     if (!b) return set_error(SCLBM_E_INVALID_ARGUMENT, "null batch");
+    if (b->use_two) { // one CTA per unit
+        if (ntiles) *ntiles = b->ntwo;
+        if (grid_ctas) *grid_ctas = b->ntwo;
+        return SCLBM_OK;
+    }
     const int r = b->use_ring == 64 ? 1 : 0;
     if (ntiles) *ntiles = b->use_ring ? b->nunits[r] : (b->use_units ? b->ntiles : batch_ntiles(b));
     if (grid_ctas)
@@ -511,8 +591,10 @@ int sclbm_batch_step(sclbm_batch *b, int nsteps, int use_graph)
             cudaGraph_t g;
             SCLBM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = cudaSuccess;
-            for (int k = 0; k < GRAPH_STEPS && e == cudaSuccess; ++k)
-                e = batch_launch_any(b, b->parity ^ (k & 1), s);
+            const int launches = b->use_two ? GRAPH_STEPS / 2 : GRAPH_STEPS; // even: the parity returns
+            for (int k = 0; k < launches && e == cudaSuccess; ++k)
+                e = b->use_two ? batch_launch_two(b, b->parity ^ (k & 1), s)
+                               : batch_launch_any(b, b->parity ^ (k & 1), s);
             cudaError_t e2 = cudaStreamEndCapture(s, &g);
             if (e != cudaSuccess) return cuda_fail(e, "batch capture");
             if (e2 != cudaSuccess) return cuda_fail(e2, "batch capture end");
@@ -523,6 +605,12 @@ int sclbm_batch_step(sclbm_batch *b, int nsteps, int use_graph)
         SCLBM_CUDA(cudaGraphLaunch(ge, s));
         done += GRAPH_STEPS; // even: parity unchanged
     }
+    // pairs in twos, so that the buffers' parity follows the steps'
+    for (; b->use_two && nsteps - done >= 4; done += 4)
+        for (int k = 0; k < 2; ++k) {
+            cudaError_t e = batch_launch_two(b, b->parity ^ k, s);
+            if (e != cudaSuccess) return cuda_fail(e, "batch step");
+        }
     for (; done < nsteps; ++done) {
         cudaError_t e = batch_launch_any(b, b->parity, s);
         if (e != cudaSuccess) return cuda_fail(e, "batch step");

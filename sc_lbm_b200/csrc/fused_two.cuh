@@ -260,27 +260,51 @@ __global__ void __launch_bounds__(TX, TWO_CTAS)
     two_unit<S, TX, FLAGS>(a, xb, min(w, a.nx - xb), y0, nrow, (band & 1) != 0, sh);
 }
 
-// Strips of one width, as few as hold the lattice.
-inline int two_strips(int nx) { return (nx + TWO_TX - 7) / (TWO_TX - 6); }
+// Width of a lattice's strips (the last one may be narrower): as few strips as
+// hold the columns, and of the widths that give as few, the one with the
+// fewest warps at work -- a strip of n columns keeps the warps of n + 6 threads
+// busy, the rest of its CTA waits at the barriers.  128 columns: 90 + 38 run
+// on five warps, 64 + 64 on six.
+inline int two_width(int nx)
+{
+    constexpr int W = TWO_TX - 6;
+    const int strips = (nx + W - 1) / W, even = (nx + strips - 1) / strips;
+    int best = even, least = 0;
+    for (int w = even; w <= W; ++w) {
+        const int warps = (nx / w) * ((w + 6 + 31) / 32) + (nx % w ? (nx % w + 6 + 31) / 32 : 0);
+        if (least == 0 || warps < least) {
+            least = warps;
+            best = w;
+        }
+    }
+    return best;
+}
 
-// Rows per band.  A band of r rows takes r + 8 iterations (six halo rows, two
-// to fill the pipeline).  With n CTAs on an SM an iteration takes as long as
-// the larger of its latency and n times a CTA's share of the SM; measured in
-// shares (0.48 us for FP32) the latency is about 1.8 of them, and four CTAs
-// are resident.  The rows with the least time over full waves and the last,
-// partial one are taken: 1024^2 16 rows (45 us a launch; 12 rows 55, 24 rows
-// 49), 256^2 3 rows (10.4; 6 rows 12.3), 4096^2 48 to 96 rows (within 2 %; 16
-// rows 8 % slower).
+// Rows per band: the relative time of `units` bands of r rows each.  A band
+// computes r + 4 rows of the first step, r of the second and takes r + 8
+// iterations, about r + 4 full ones; four CTAs are resident per SM and a full
+// wave of them takes four shares of an SM's throughput per iteration.  In the
+// last, partial wave an iteration with n CTAs on an SM takes longer than n
+// shares, down to the latency of one (measured with solid nodes, where a share
+// is 0.66 us: 1.6, 1.9, 2.45 and 2.9 us for one to four).  Measured by this
+// choice / other heights, us per step: 1021 x 763 12 rows 21.9 / 8 rows 25.0,
+// 24 rows 23.6; 1024^2 16 rows 22.6 / 12 rows 26.0, 24 rows 24.7; 256^2 3 rows
+// 5.4 / 6 rows 6.2; a batch of eight 400 x 306 20 rows 35.9 / 16 rows 49.5, 6
+// rows 39.3; 4096^2 within 2 % from 48 to 96 rows.
+constexpr int TWO_ROWS[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64};
+inline double two_cost(long units, int r, int sms)
+{
+    const double last[TWO_CTAS + 1] = {0.0, 2.4, 2.9, 3.7, 4.2};
+    const long wave = (long)TWO_CTAS * sms, rest = units % wave;
+    return (r + 4) * ((double)(units / wave) * TWO_CTAS + last[(rest + sms - 1) / sms]);
+}
 inline int two_rows(int nx, int ny, int sms)
 {
-    const int cand[] = {2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 56, 64};
-    int best = 2;
+    const int w = two_width(nx), strips = (nx + w - 1) / w;
+    int best = 1;
     double least = 0.0;
-    for (int r : cand) {
-        const long units = (long)two_strips(nx) * ((ny + r - 1) / r), wave = (long)TWO_CTAS * sms;
-        const long rest = units % wave;
-        const double last = rest ? std::max(1.8, (double)((rest + sms - 1) / sms)) : 0.0;
-        const double cost = (r + 8) * ((double)(units / wave) * TWO_CTAS + last);
+    for (int r : TWO_ROWS) {
+        const double cost = two_cost((long)strips * ((ny + r - 1) / r), r, sms);
         if (least == 0.0 || cost < least) {
             least = cost;
             best = r;
@@ -292,8 +316,7 @@ inline int two_rows(int nx, int ny, int sms)
 template <typename S, int TX, int FLAGS>
 inline cudaError_t launch_two2_f(const Fused2Args<S, float> &a, int rows, cudaStream_t s)
 {
-    const int strips = two_strips(a.nx);
-    const int w = (a.nx + strips - 1) / strips;
+    const int w = two_width(a.nx), strips = (a.nx + w - 1) / w;
     const int bands = std::min((a.ny + rows - 1) / rows, 65535);
     k_two2<S, TX, FLAGS><<<dim3(strips, bands), TX, 0, s>>>(a, w, bands);
     return cudaGetLastError();
@@ -313,6 +336,48 @@ inline cudaError_t launch_two2_any(const Fused2Args<S, float> &a, int rows, cuda
     case KF_SOLID: return launch_two2_f<S, TWO_TX, KF_SOLID | KF_UNIFORM>(a, rows, s);
     default: return launch_two2_f<S, TWO_TX, KF_FORCE | KF_SOLID | KF_UNIFORM>(a, rows, s);
     }
+}
+
+// ---------------------------------------------------------------- batches
+// A unit of the batched kernel: the columns [xb, xb + ncol) and rows
+// [y0, y0 + nrow) of domain dom; down: the march direction (alternating
+// between a domain's bands).
+struct TwoUnit {
+    int dom, xb, ncol, y0, nrow, down;
+};
+
+// One CTA per unit, in the list's order (largest first): the block scheduler
+// balances them, no counter to take turns at.  doms holds two entries per
+// domain (buffer parity 0 and 1); the unit's argument block is copied into
+// shared memory.
+template <typename S, int FLAGS>
+__global__ void __launch_bounds__(TWO_TX, TWO_CTAS)
+    k_batch_two(const Fused2Args<S, float> *__restrict__ doms, const TwoUnit *__restrict__ units, int parity)
+{
+    __shared__ TwoShared<S, TWO_TX> sh;
+    __shared__ __align__(16) Fused2Args<S, float> sa;
+    static_assert(sizeof(sa) % 4 == 0, "argument block copied as words");
+    const TwoUnit u = units[blockIdx.x];
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(doms + 2 * u.dom + parity);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(&sa);
+    for (int w = threadIdx.x; w < (int)(sizeof(sa) / 4); w += TWO_TX) dst[w] = src[w];
+    __syncthreads();
+    two_unit<S, TWO_TX, FLAGS>(sa, u.xb, u.ncol, u.y0, u.nrow, u.down != 0, sh);
+}
+
+// flags: KF_FORCE / KF_SOLID when any domain of the batch has a volume force /
+// a solid node
+template <typename S>
+inline cudaError_t launch_batch_two_any(const Fused2Args<S, float> *doms, const TwoUnit *units, int nunits,
+                                        int parity, int flags, cudaStream_t s)
+{
+    if (flags & KF_SOLID)
+        k_batch_two<S, KF_FORCE | KF_SOLID | KF_UNIFORM><<<nunits, TWO_TX, 0, s>>>(doms, units, parity);
+    else if (flags & KF_FORCE)
+        k_batch_two<S, KF_FORCE><<<nunits, TWO_TX, 0, s>>>(doms, units, parity);
+    else
+        k_batch_two<S, 0><<<nunits, TWO_TX, 0, s>>>(doms, units, parity);
+    return cudaGetLastError();
 }
 
 } // namespace sclbm

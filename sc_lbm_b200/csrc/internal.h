@@ -203,6 +203,11 @@ constexpr int ASYNC_STRIP = 128;
 // the state two steps later; rows per band (0 default)
 cudaError_t launch_two2_f32(const Fused2Args<float, float> &a, int rows, cudaStream_t s);
 cudaError_t launch_two2_f16(const Fused2Args<__half, float> &a, int rows, cudaStream_t s);
+struct TwoUnit;
+cudaError_t launch_batch_two_f32(const Fused2Args<float, float> *doms, const TwoUnit *units, int nunits,
+                                 int parity, int flags, cudaStream_t s);
+cudaError_t launch_batch_two_f16(const Fused2Args<__half, float> *doms, const TwoUnit *units, int nunits,
+                                 int parity, int flags, cudaStream_t s);
 // density pass (kernel a): rho (or rho - rho_ref for shifted storage) per node,
 // 0 at solid nodes; both components in one launch
 cudaError_t launch_density_fp64(const uint8_t *mask, const double *f0, const double *f1,

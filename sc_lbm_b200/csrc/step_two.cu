@@ -12,5 +12,15 @@ cudaError_t launch_two2_f16(const Fused2Args<__half, float> &a, int rows, cudaSt
 {
     return launch_two2_any(a, rows, s);
 }
+cudaError_t launch_batch_two_f32(const Fused2Args<float, float> *doms, const TwoUnit *units, int nunits,
+                                 int parity, int flags, cudaStream_t s)
+{
+    return launch_batch_two_any(doms, units, nunits, parity, flags, s);
+}
+cudaError_t launch_batch_two_f16(const Fused2Args<__half, float> *doms, const TwoUnit *units, int nunits,
+                                 int parity, int flags, cudaStream_t s)
+{
+    return launch_batch_two_any(doms, units, nunits, parity, flags, s);
+}
 
 } // namespace sclbm

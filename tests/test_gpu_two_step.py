@@ -88,3 +88,22 @@ def test_captured_steps_replay(sclbm):
     finally:
         sclbm.synchronize()
         sclbm.set_stream(None)
+
+
+@pytest.mark.parametrize("prec_name", ["FP32_SHIFTED", "FP16_SHIFTED"])
+@pytest.mark.parametrize("porous", [False, True])
+def test_batch_pairs_match_single_steps(sclbm, prec_name, porous):
+    """Uneven domains, a caller's band height, runs of whole graphs and of a few steps."""
+    prec = getattr(sclbm, prec_name)
+    sizes = [(4, 4), (64, 33), (128, 70), (130, 17), (245, 31), (512, 9)]
+    build = [make(sclbm, nx, ny, prec, porous, k % 2 == 1, seed=9 + k) for k, (nx, ny) in enumerate(sizes)]
+    alone = [b(2) for b in build]
+    for a in alone:
+        a.step(27)
+    for tile_y in (None, [7] * len(sizes)):
+        doms = [b() for b in build]
+        batch = sclbm.Batch(doms, tile_y)
+        batch.step(1)
+        batch.step(26)
+        for d, a, size in zip(doms, alone, sizes):
+            assert state(d) == state(a), (size, tile_y)
