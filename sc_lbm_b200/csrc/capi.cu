@@ -781,7 +781,10 @@ int sclbm_lbm_step(sclbm_lbm *l, const sclbm_geometry *g, sclbm_fluid *f1, sclbm
         a.fin[1] = f2->d[SCLBM_FIELD_F];
         a.fout[0] = l->d_tmp[0];
         a.fout[1] = l->d_tmp[1];
-        CUDA_LAUNCH(launch_fused2_async_fp64(a, stream()));
+        // one node per thread up to 4 M nodes (520 x 260: 9.0 us a step against
+        // 19.0), the pipelined kernel beyond
+        CUDA_LAUNCH(a.N < ((size_t)1 << 22) && flat_fits(g->nx, g->ny) ? launch_flat2_fp64(a, stream())
+                                                                    : launch_fused2_async_fp64(a, stream()));
         std::swap(f1->d[SCLBM_FIELD_F], l->d_tmp[0]);
         std::swap(f2->d[SCLBM_FIELD_F], l->d_tmp[1]);
     }

@@ -334,6 +334,15 @@ static bool ring_fills_device(const sclbm_domain *d)
     return units >= 3 * per_sm * sm_count();
 }
 
+// Lattices on which one node per thread is faster than the ring although the
+// ring's bands fill the GPU: FP64 up to 4 M nodes (1500^2 113 us against 125,
+// 2048^2 210 against 205, with solid nodes 251 against 258; 4096 x 2048 438
+// against 387).  FP32 and FP16 rings start at 5 and 7 M nodes, far beyond L2.
+static bool flat_beats_ring(const sclbm_domain *d)
+{
+    return d->prec == SCLBM_FP64 && d->N < ((size_t)1 << 22);
+}
+
 template <typename S, typename T>
 static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
 {
@@ -365,14 +374,23 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
                                    (float *)d->rho_tmp[1], d->N, s);
         if (e != cudaSuccess) return e;
     }
-    // variant 0 picks the fastest measured form on B200: the ring kernel
-    // (rows streamed into shared memory by tensor copies) at the depth and
-    // band height of ring_choice on lattices whose rows start on 16-byte
-    // boundaries and whose bands fill three waves; else the register tile,
-    // in its uniform solid form where FP32/FP16 lattices have solid nodes.
-    // 3 and 9 force the pipelined kernel; 11, 12, 13 the ring kernel with its
-    // default, fewer and more stages (unaligned lattices: the register tile)
-    if (d->variant == 0 && ring_row_aligned(d) && ring_fills_device(d)) {
+    // variant 0 picks the fastest measured form on B200: one node per thread,
+    // or the ring kernel (rows streamed into shared memory by tensor copies)
+    // at the depth and band height of ring_choice on large lattices whose rows
+    // start on 16-byte boundaries.  A tile height or width of the caller's
+    // choice asks for marching tiles: the ring where it fits and fills the
+    // GPU, else the register tile, in its uniform solid form where FP32/FP16
+    // lattices have solid nodes.  3 and 9 force the pipelined kernel; 11, 12,
+    // 13 the ring kernel with its default, fewer and more stages (unaligned
+    // lattices: the register tile)
+    const bool ring = d->variant == 0 && ring_row_aligned(d) && ring_fills_device(d);
+    if (d->variant == 0 && d->tile_y == 0 && d->tx == 128 && flat_fits(d->nx, d->ny) &&
+        (!ring || flat_beats_ring(d))) {
+        if constexpr (sizeof(S) == 8) return launch_flat2_fp64(a, s);
+        else if constexpr (sizeof(S) == 4) return launch_flat2_f32(a, s);
+        else return launch_flat2_f16(a, s);
+    }
+    if (ring) {
         const RingChoice rc = ring_choice(d);
         const int rows = d->tile_y > 0 ? d->tile_y : rc.rows;
         if constexpr (sizeof(S) == 8) return launch_ring2_fp64(a, rc.stages, rows, s);
@@ -412,16 +430,19 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
     else return launch_fused2_f16(a, v, d->tx, s);
 }
 
-// Whether the domain's steps run in pairs (fused_two.cuh), which is faster at
-// every size of the shifted forms: FP32 256^2 5.4 us a step against 8.2, 1024^2
-// 22.6 against 35.5, 4096^2 270 against 407.  Lattices that need 64-bit
-// offsets or that a halo of three wraps around more than once, and domains
-// with a variant or a tile width of the caller's choice, keep the one-step
-// kernels.
+// Whether the domain's steps run in pairs (fused_two.cuh): the shifted forms
+// beyond 600 k (FP32) or 1.1 M (FP16) nodes, where both buffers outgrow L2;
+// below, one node per thread is faster.  us per step, pairs / one node per
+// thread: FP32 512^2 9.3 / 7.5, 768^2 15.4 / 15.4 (with solid nodes 18.9 /
+// 18.7), 1024^2 22.6 / 31.6; FP16 768^2 17.5 / 14.3, 1024^2 24.6 / 24.0 (29.9 /
+// 28.5), 2048 x 1024 44 / 47.5.  Lattices that need 64-bit offsets, and domains
+// with a variant or a tile width of the caller's choice, take single steps; a
+// band height of the caller's choice asks for pairs.
 static bool two_step(const sclbm_domain *d)
 {
+    const size_t most = d->prec == SCLBM_FP32_SHIFTED ? 600000 : 1100000;
     return d->variant == 0 && d->tx == 128 && d->ncomp == 2 && d->prec != SCLBM_FP64 && d->nx >= 4 &&
-           d->ny >= 4 && !needs_wide_offsets(d->N);
+           d->ny >= 4 && (d->tile_y > 0 || d->N > most) && !needs_wide_offsets(d->N);
 }
 
 // whether work queued on s goes into a graph (or cannot be told not to)

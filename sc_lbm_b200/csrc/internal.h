@@ -199,6 +199,12 @@ int ring_maps_of(const Fused2Args<__half, float> &a, int width, RingMaps *m);
 int async_resident_fp64(); // CTAs of the batched kernel resident on the device
 int async_resident_f32();
 constexpr int ASYNC_STRIP = 128;
+// one step, one node per thread (fused_flat.cuh); lattices for which flat_fits
+// is false are refused with cudaErrorInvalidValue
+bool flat_fits(size_t nx, size_t ny);
+cudaError_t launch_flat2_fp64(const Fused2Args<double, double> &a, cudaStream_t s);
+cudaError_t launch_flat2_f32(const Fused2Args<float, float> &a, cudaStream_t s);
+cudaError_t launch_flat2_f16(const Fused2Args<__half, float> &a, cudaStream_t s);
 // two steps in one launch (fused_two.cuh): fin holds the state, fout receives
 // the state two steps later; rows per band (0 default)
 cudaError_t launch_two2_f32(const Fused2Args<float, float> &a, int rows, cudaStream_t s);

@@ -1,6 +1,7 @@
-"""Steps run in pairs (two per launch) against the one-step register tile.
+"""The default step kernels -- one node per thread, and steps run in pairs (two
+per launch) -- against the register tile.
 
-The pair kernel's nodes run the same arithmetic as the one-step kernels' and
+Their nodes run the same arithmetic as the register tile's, and pairs
 hold the state between the steps in the storage type, so the populations are
 equal byte for byte: at widths around its strips (122 columns), with bands of
 one row and of uneven heights, on lattices that its halo wraps around, for odd
@@ -25,7 +26,7 @@ def make(sclbm, nx, ny, prec, porous, force, seed=5):
 
     def build(variant=0, rows=0):
         d = sclbm.Domain(nx, ny, mask, p, prec)
-        d.set_kernel(variant, rows)
+        d.set_kernel(variant, rows)  # a band height asks for pairs
         for k in range(2):
             d.upload_f(k, f[k])
         return d
@@ -37,8 +38,8 @@ def state(d):
 
 
 @pytest.mark.parametrize("prec_name", ["FP32_SHIFTED", "FP16_SHIFTED"])
-@pytest.mark.parametrize("nx,ny,rows", [(4, 4, 0), (5, 7, 1), (64, 33, 5), (121, 20, 0), (122, 9, 4),
-                                        (123, 40, 32), (245, 31, 0), (1021, 77, 7)])
+@pytest.mark.parametrize("nx,ny,rows", [(4, 4, 2), (5, 7, 1), (64, 33, 5), (121, 20, 20), (122, 9, 4),
+                                        (123, 40, 32), (245, 31, 3), (1021, 77, 7), (1200, 1000, 0)])
 def test_pairs_match_single_steps(sclbm, prec_name, nx, ny, rows):
     prec = getattr(sclbm, prec_name)
     for porous in (False, True):
@@ -51,10 +52,26 @@ def test_pairs_match_single_steps(sclbm, prec_name, nx, ny, rows):
                 assert state(a) == state(b), (porous, force, steps)
 
 
+@pytest.mark.parametrize("prec_name", ["FP64", "FP32_SHIFTED", "FP16_SHIFTED"])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (1, 9), (7, 1), (31, 3), (32, 4), (33, 5), (64, 37), (129, 130)])
+def test_one_node_per_thread_matches_tiles(sclbm, prec_name, nx, ny):
+    """Tiles of 32 x 4 nodes: full, partial and wrapping around the lattice."""
+    prec = getattr(sclbm, prec_name)
+    for porous in (False, True):
+        for force in (False, True):
+            build = make(sclbm, nx, ny, prec, porous, force)
+            a, b = build(), build(2)
+            a.step(5)
+            b.step(5)
+            assert state(a) == state(b), (porous, force)
+
+
 def test_pairs_keep_a_domain_in_step_with_its_batch(sclbm):
     """Two steps outside the batch leave it usable, one does not."""
     build = [make(sclbm, nx, 48, sclbm.FP32_SHIFTED, True, False) for nx in (96, 60)]
     doms, alone = [b() for b in build], [b(2) for b in build]
+    for d in doms:
+        d.set_kernel(0, 16)
     doms[0].step(2)  # before the batch takes the buffers' addresses
     batch = sclbm.Batch(doms)
     doms[1].step(6)
@@ -68,7 +85,8 @@ def test_pairs_keep_a_domain_in_step_with_its_batch(sclbm):
         batch.step(1)
 
 
-def test_captured_steps_replay(sclbm):
+@pytest.mark.parametrize("rows", [0, 16])
+def test_captured_steps_replay(sclbm, rows):
     import torch
     build = make(sclbm, 130, 50, sclbm.FP32_SHIFTED, False, True)
     d, one = build(), build(2)
@@ -76,6 +94,7 @@ def test_captured_steps_replay(sclbm):
     sclbm.synchronize()
     sclbm.set_stream(st.cuda_stream)
     try:
+        d.set_kernel(0, rows)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g, stream=st):
             d.step(6)
