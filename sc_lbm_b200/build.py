@@ -25,7 +25,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
           f"-I{os.path.join(ROOT, 'include')}", f"-I{os.path.join(HOST, 'include')}", f"-I{GEN}"]
-EXACT = {"ops_fp64.cu", "step_flat64.cu"}
+EXACT = {"ops_fp64.cu", "step_flat64.cu", "step_single64.cu"}
 PRECISIONS = ("fp64", "fp32s", "fp16s")  # sclbm_precision order
 
 

@@ -62,6 +62,16 @@ int ensure_device()
     return SCLBM_OK;
 }
 
+bool being_captured(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 cudaStream_t stream() { return g_user_set ? g_user_stream : g_own_stream; }
 int sm_count() { return g_sms > 0 ? g_sms : 148; }
 
@@ -808,10 +818,16 @@ int sclbm_lbm_step_single(sclbm_lbm *l, const sclbm_geometry *g, sclbm_fluid *f,
     a.c.inv_omega = 1.0 / f->omega;
     a.c.force_on = force != nullptr;
     for (int i = 0; i < 9; ++i) a.c.force[i] = force ? force[i] : 0.0;
-    for (int s = 0; s < nsteps; ++s) {
+    // several steps per launch; under capture odd ones, so that the arrays end
+    // where single steps would leave them
+    const bool several = single_fits(g->nx, g->ny), odd = several && being_captured(stream());
+    const int K = several ? single_depth(g->nx, g->ny, true) : 1;
+    for (int s = 0, n; s < nsteps; s += n) {
+        n = std::min(K, nsteps - s);
+        if (odd && n % 2 == 0) --n;
         a.fin = f->d[SCLBM_FIELD_F];
         a.fout = l->d_tmp[0];
-        CUDA_LAUNCH(launch_fused1_fp64(a, stream()));
+        CUDA_LAUNCH(several ? launch_single_fp64(a, K, n, stream()) : launch_fused1_fp64(a, stream()));
         std::swap(f->d[SCLBM_FIELD_F], l->d_tmp[0]);
     }
     return SCLBM_OK;

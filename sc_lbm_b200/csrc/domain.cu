@@ -289,6 +289,19 @@ static void fill2(const sclbm_domain *d, Fused2Args<S, T> &a)
     a.status = d->d_status;
 }
 
+template <typename S, typename T>
+static void fill1(const sclbm_domain *d, Fused1Args<S, T> &a)
+{
+    a = Fused1Args<S, T>{};
+    a.nx = (int)d->nx;
+    a.ny = (int)d->ny;
+    a.N = d->N;
+    a.mask = d->d_mask;
+    a.fin = (const S *)d->buf[d->parity][0];
+    a.fout = (S *)d->buf[d->parity ^ 1][0];
+    fill_comp<T>(a.c, d->p, 0);
+}
+
 void domain_fused2_args(const sclbm_domain *d, Fused2Args<double, double> *a64,
                         Fused2Args<float, float> *a32, Fused2Args<__half, float> *a16)
 {
@@ -347,14 +360,8 @@ template <typename S, typename T>
 static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
 {
     if (d->ncomp == 1) {
-        Fused1Args<S, T> a{};
-        a.nx = (int)d->nx;
-        a.ny = (int)d->ny;
-        a.N = d->N;
-        a.mask = d->d_mask;
-        a.fin = (const S *)d->buf[d->parity][0];
-        a.fout = (S *)d->buf[d->parity ^ 1][0];
-        fill_comp<T>(a.c, d->p, 0);
+        Fused1Args<S, T> a;
+        fill1(d, a);
         if constexpr (sizeof(S) == 8) return launch_fused1_fp64(a, s);
         else if constexpr (sizeof(S) == 4) return launch_fused1_f32(a, s);
         else return launch_fused1_f16(a, s);
@@ -445,17 +452,6 @@ static bool two_step(const sclbm_domain *d)
            d->ny >= 4 && (d->tile_y > 0 || d->N > most) && !needs_wide_offsets(d->N);
 }
 
-// whether work queued on s goes into a graph (or cannot be told not to)
-static bool being_captured(cudaStream_t s)
-{
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-        cudaGetLastError();
-        return true;
-    }
-    return st != cudaStreamCaptureStatusNone;
-}
-
 // two steps in one launch
 static int domain_launch_two(sclbm_domain *d, cudaStream_t s)
 {
@@ -472,6 +468,46 @@ static int domain_launch_two(sclbm_domain *d, cudaStream_t s)
     if (e != cudaSuccess) return cuda_fail(e, "two-step launch");
     d->parity ^= 1;
     return SCLBM_OK;
+}
+
+// nsteps of a single-component domain, several per launch
+static int domain_single_steps(sclbm_domain *d, int nsteps, cudaStream_t s)
+{
+    const int K = single_depth(d->nx, d->ny, d->prec == SCLBM_FP64);
+    // a graph has to find the state where it left it: odd launches turn the
+    // buffers over as often as their steps would
+    const bool odd = being_captured(s);
+    int rc = SCLBM_OK, done = 0, launches = 0;
+    while (done < nsteps) {
+        int n = std::min(K, nsteps - done);
+        if (odd && n % 2 == 0) --n;
+        cudaError_t e;
+        if (d->prec == SCLBM_FP64) {
+            Fused1Args<double, double> a;
+            fill1(d, a);
+            e = launch_single_fp64(a, K, n, s);
+        } else if (d->prec == SCLBM_FP32_SHIFTED) {
+            Fused1Args<float, float> a;
+            fill1(d, a);
+            e = launch_single_f32(a, K, n, s);
+        } else {
+            Fused1Args<__half, float> a;
+            fill1(d, a);
+            e = launch_single_f16(a, K, n, s);
+        }
+        if (e != cudaSuccess) {
+            rc = cuda_fail(e, "single-component step launch");
+            break;
+        }
+        d->parity ^= 1;
+        done += n;
+        ++launches;
+    }
+    if ((done ^ launches) & 1) { // the parity counts steps
+        std::swap(d->buf[0], d->buf[1]);
+        d->parity ^= 1;
+    }
+    return rc;
 }
 
 int domain_launch_step(sclbm_domain *d, cudaStream_t s)
@@ -859,6 +895,7 @@ int sclbm_domain_step(sclbm_domain *d, int nsteps)
     if (d->variant == 1 && d->ncomp == 2 && !d->rho_tmp[0])
         return set_error(SCLBM_E_RUNTIME, "two-pass buffers missing");
     cudaStream_t s = stream();
+    if (d->ncomp == 1 && single_fits(d->nx, d->ny)) return domain_single_steps(d, nsteps, s);
     int rc = SCLBM_OK, pairs = two_step(d) ? nsteps / 2 : 0;
     // The parity counts steps (a batch's domains have to be in step), and a pair
     // turns the buffers over once: after an odd number of pairs the two buffers

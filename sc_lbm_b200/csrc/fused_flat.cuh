@@ -15,9 +15,7 @@
 // The arithmetic per node is collide_push's, so the results equal the other
 // kernels' byte for byte.
 //
-// The kernel is launched as a programmatic dependent of the one before it in
-// the stream: its CTAs take their places while that one drains and wait for
-// its end before the first access to memory.
+// The kernel is launched as a programmatic dependent (launch.cuh).
 //
 // Measured on one B200, us per step (before: register tile or pipelined
 // kernel): FP64 64^2 4.0 (10.3), 256^2 5.4 (12.3), 512^2 12.3 (18.5), 1024^2
@@ -25,44 +23,9 @@
 // (87), 130 (150); FP32 256^2 3.5 (8.2), 512^2 7.5 (12.3); FP16 1024^2 24 (32).
 #pragma once
 #include "fused_step.cuh"
+#include "launch.cuh"
 
 namespace sclbm {
-
-// everything the previous kernel of the stream wrote is visible after this
-__device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// the next kernel of the stream may take its places from here on
-__device__ __forceinline__ void dependent_launch()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-// ordinary loads (the read-only path may hold lines from before the wait)
-template <typename S> struct Load {
-    static __device__ __forceinline__ S value(const S *p) { return *p; }
-};
-template <> struct Load<__half> {
-    static __device__ __forceinline__ float value(const __half *p) { return __half2float(*p); }
-};
-
-// Launches kern as a programmatic dependent of the previous kernel in the
-// stream: it may start before that one has ended and calls dependent_wait
-// before it touches memory.  It calls dependent_launch after the wait, so at
-// most two kernels of a chain are under way and the one before them has ended:
-// with two buffers in turn, nothing that a kernel writes is still being read.
-template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t s, A &&...args)
-{
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c{};
-    c.gridDim = grid;
-    c.blockDim = block;
-    c.stream = s;
-    c.attrs = &at;
-    c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kern, std::forward<A>(args)...);
-}
 
 constexpr int FLAT_ROWS = 4;
 
@@ -101,7 +64,7 @@ __global__ void __launch_bounds__(32 * TY, (flat_ctas<T>()))
         halo = u < 2 * TY && hr <= nrow;
     }
     dependent_wait();
-    dependent_launch(); // after the wait: see launch_dependent
+    dependent_launch();
     T f[2][9], h[2][9];
     uint8_t m = 1, mh = 1;
     const uint32_t node = (uint32_t)y * (uint32_t)nx + (uint32_t)x;
@@ -146,10 +109,10 @@ inline cudaError_t launch_flat2_any(const Fused2Args<S, T> &a, cudaStream_t s)
     if (!flat_fits(a.nx, a.ny)) return cudaErrorInvalidValue;
     const dim3 grid((a.nx + 31) / 32, (a.ny + TY - 1) / TY), block(32 * TY);
     switch (kernel_flags(a)) {
-    case 0: return launch_dependent(k_flat2<S, T, TY, 0>, grid, block, s, a);
-    case KF_FORCE: return launch_dependent(k_flat2<S, T, TY, KF_FORCE>, grid, block, s, a);
-    case KF_SOLID: return launch_dependent(k_flat2<S, T, TY, KF_SOLID | UNI>, grid, block, s, a);
-    default: return launch_dependent(k_flat2<S, T, TY, KF_FORCE | KF_SOLID | UNI>, grid, block, s, a);
+    case 0: return launch_dependent(k_flat2<S, T, TY, 0>, grid, block, 0, s, a);
+    case KF_FORCE: return launch_dependent(k_flat2<S, T, TY, KF_FORCE>, grid, block, 0, s, a);
+    case KF_SOLID: return launch_dependent(k_flat2<S, T, TY, KF_SOLID | UNI>, grid, block, 0, s, a);
+    default: return launch_dependent(k_flat2<S, T, TY, KF_FORCE | KF_SOLID | UNI>, grid, block, 0, s, a);
     }
 }
 

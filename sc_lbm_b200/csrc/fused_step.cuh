@@ -63,6 +63,15 @@ template <> struct Store<__half> {
     static __device__ __forceinline__ void st(__half *p, float v) { *p = __float2half_rn(v); }
 };
 
+// ordinary loads, in the compute type (Store::ld takes the read-only path,
+// which kernels launched as programmatic dependents leave: launch.cuh)
+template <typename S> struct Load {
+    static __device__ __forceinline__ S value(const S *p) { return *p; }
+};
+template <> struct Load<__half> {
+    static __device__ __forceinline__ float value(const __half *p) { return __half2float(*p); }
+};
+
 // Bulk prefetch of [p, p + bytes) into L2 (p and bytes multiples of 16): one
 // instruction brings a whole row segment of a population array closer before
 // the per-thread loads of a later row iteration ask for it.
@@ -945,10 +954,53 @@ __global__ void __launch_bounds__(TX, (fused_min_ctas<T, AHEAD, FLAGS, TX>()))
 // single-component fused step: collide(geom,f) + add_volume_force + stream
 // (src/lbm.cpp:275-288, 315-325, 343-384; src/fluid.cpp:175-243)
 // ---------------------------------------------------------------------------
+// post-collision populations of one node
+template <typename S, typename T>
+__device__ __forceinline__ void collide_single(const CompParams<T> &c, const T (&f)[9], T (&out)[9])
+{
+    if constexpr (sizeof(T) == 8) {
+        double r = 0.0, ux = 0.0, uy = 0.0;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) r += f[i];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            ux += f[i] * double(cx(i));
+            uy += f[i] * double(cy(i));
+        }
+        ux /= r;
+        uy /= r;
+        double fe[9];
+        feq_exact(r, ux, uy, fe);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            double v = c.one_m_omega * f[i] + c.omega * fe[i];
+            if (c.force_on) v += c.force[i];
+            out[i] = v;
+        }
+    } else {
+        float dr = 0.f;
+#pragma unroll
+        for (int i = 0; i < 9; ++i) dr += f[i];
+        const float r = c.rho_ref + dr;
+        const float jx = (f[1] - f[3]) + (f[5] - f[6]) + (f[8] - f[7]);
+        const float jy = (f[2] - f[4]) + (f[5] + f[6]) - (f[7] + f[8]);
+        const float ir = 1.0f / r;
+        const float ux = jx * ir, uy = jy * ir;
+        const float usq15 = 1.5f * fmaf(ux, ux, uy * uy);
+#pragma unroll
+        for (int i = 1; i < 9; ++i) {
+            float v = fmaf(c.omega, feq_dev(i, dr, r, ux, uy, usq15) - f[i], f[i]);
+            if (c.force_on) v += c.force[i];
+            out[i] = stored_value<S>(v);
+        }
+        // the rest population closes the node's mass (see mass_closing_rest)
+        out[0] = mass_closing_rest(f, out, c.force_on ? c.force_sum : 0.f);
+    }
+}
+
 template <typename S, typename T>
 __global__ void __launch_bounds__(256) k_fused1(const Fused1Args<S, T> a)
 {
-    constexpr bool EXACT = sizeof(T) == 8;
     const size_t N = a.N;
     const int nx = a.nx, ny = a.ny;
     for (size_t node = blockIdx.x * (size_t)blockDim.x + threadIdx.x; node < N;
@@ -964,47 +1016,7 @@ __global__ void __launch_bounds__(256) k_fused1(const Fused1Args<S, T> a)
 #pragma unroll
         for (int i = 0; i < 9; ++i) f[i] = T(Store<S>::ld(a.fin + i * N + node));
         T out[9];
-        if constexpr (EXACT) {
-            double r = 0.0, ux = 0.0, uy = 0.0;
-#pragma unroll
-            for (int i = 0; i < 9; ++i) r += f[i];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                ux += f[i] * double(cx(i));
-                uy += f[i] * double(cy(i));
-            }
-            ux /= r;
-            uy /= r;
-            double fe[9];
-            feq_exact(r, ux, uy, fe);
-#pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                double v = a.c.one_m_omega * f[i] + a.c.omega * fe[i];
-                if (a.c.force_on) v += a.c.force[i];
-                out[i] = v;
-            }
-        } else {
-            float dr = 0.f;
-#pragma unroll
-            for (int i = 0; i < 9; ++i) dr += f[i];
-            const float r = a.c.rho_ref + dr;
-            const float jx = (f[1] - f[3]) + (f[5] - f[6]) + (f[8] - f[7]);
-            const float jy = (f[2] - f[4]) + (f[5] + f[6]) - (f[7] + f[8]);
-            const float ir = 1.0f / r;
-            const float ux = jx * ir, uy = jy * ir;
-            const float usq15 = 1.5f * fmaf(ux, ux, uy * uy);
-            float v[9];
-#pragma unroll
-            for (int i = 1; i < 9; ++i) {
-                v[i] = fmaf(a.c.omega, feq_dev(i, dr, r, ux, uy, usq15) - f[i], f[i]);
-                if (a.c.force_on) v[i] += a.c.force[i];
-                v[i] = stored_value<S>(v[i]);
-            }
-            // the rest population closes the node's mass (see mass_closing_rest)
-            v[0] = mass_closing_rest(f, v, a.c.force_on ? a.c.force_sum : 0.f);
-#pragma unroll
-            for (int i = 0; i < 9; ++i) out[i] = v[i];
-        }
+        collide_single<S, T>(a.c, f, out);
         const int xl = wrap1(x - 1, nx), xr = wrap1(x + 1, nx);
         const int yd = wrap1(y - 1, ny), yu = wrap1(y + 1, ny);
         Store<S>::st(a.fout + node, out[0]);

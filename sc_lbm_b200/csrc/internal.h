@@ -32,6 +32,7 @@ cudaStream_t stream();
 int ensure_device();
 int grid_for(size_t n, int block);  // grid-stride grid size (multiple of the SM count)
 int sm_count();
+bool being_captured(cudaStream_t s); // work queued on s goes into a graph, or cannot be told not to
 
 // ------------------------------------------------------------- host geometry
 int geom_add_walls(std::vector<int32_t> &g, size_t nx, size_t ny, size_t dH, const std::string &w);
@@ -205,6 +206,13 @@ bool flat_fits(size_t nx, size_t ny);
 cudaError_t launch_flat2_fp64(const Fused2Args<double, double> &a, cudaStream_t s);
 cudaError_t launch_flat2_f32(const Fused2Args<float, float> &a, cudaStream_t s);
 cudaError_t launch_flat2_f16(const Fused2Args<__half, float> &a, cudaStream_t s);
+// `steps` <= K single-component steps in one launch (fused_single.cuh), K from
+// single_depth; lattices for which single_fits is false are refused
+bool single_fits(size_t nx, size_t ny);
+int single_depth(size_t nx, size_t ny, bool fp64);
+cudaError_t launch_single_fp64(const Fused1Args<double, double> &a, int K, int steps, cudaStream_t s);
+cudaError_t launch_single_f32(const Fused1Args<float, float> &a, int K, int steps, cudaStream_t s);
+cudaError_t launch_single_f16(const Fused1Args<__half, float> &a, int K, int steps, cudaStream_t s);
 // two steps in one launch (fused_two.cuh): fin holds the state, fout receives
 // the state two steps later; rows per band (0 default)
 cudaError_t launch_two2_f32(const Fused2Args<float, float> &a, int rows, cudaStream_t s);

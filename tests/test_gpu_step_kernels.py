@@ -126,3 +126,51 @@ def test_batch_pairs_match_single_steps(sclbm, prec_name, porous):
         batch.step(26)
         for d, a, size in zip(doms, alone, sizes):
             assert state(d) == state(a), (size, tile_y)
+
+
+@pytest.mark.parametrize("prec_name", ["FP64", "FP32_SHIFTED", "FP16_SHIFTED"])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (1, 9), (7, 1), (22, 6), (23, 13), (64, 33), (400, 180), (420, 200),
+                                   (700, 333)])
+def test_single_component_steps_per_launch(sclbm, prec_name, nx, ny):
+    """K steps in one launch (K = 6, 5, 3 or 2 by size) against K calls of one
+    step, whose tiles hold the halo but use one node of it."""
+    from sc_lbm_b200 import workloads as W
+    n = nx * ny
+    for porous in (False, True):
+        mask = (W.uniform(3, n) < 0.75).astype(np.int32) if porous else np.ones(n, np.int32)
+        p = sclbm.make_params(ncomp=1, tau=(0.9, 1.0), force=(W.force_vec(1e-5, "x") if porous else None, None))
+        f = W.populations(1 + 0.1 * (2 * W.uniform(4, n) - 1), mask)
+        out = []
+        for calls in ([13], [1] * 13, [2, 5, 6]):
+            d = sclbm.Domain(nx, ny, mask, p, getattr(sclbm, prec_name))
+            d.upload_f(0, f)
+            for k in calls:
+                d.step(k)
+            out.append(d.download_f(0).tobytes())
+        assert out[0] == out[1] == out[2], porous
+
+
+def test_single_component_matches_reference_steps(sclbm):
+    """FP64, a wall, random solids and a force, at sizes around the tiles."""
+    from sc_lbm_b200 import workloads as W
+    for nx, ny in ((3, 2), (23, 7), (45, 30), (120, 50)):
+        n = nx * ny
+        mask = (W.uniform(nx, n) < 0.8).astype(np.int32)
+        mask[:nx] = 0
+        F = W.force_vec(1e-4, "x")
+        g = sclbm.Geometry.from_mask(nx, ny, mask)
+        fl, lbm = sclbm.Fluid(g, 0.8), sclbm.LBM(g)
+        f = W.populations(1 + 0.1 * (2 * W.uniform(5, n) - 1), mask)
+        fl.set("f", f)
+        for _ in range(9):  # the reference's operators, one call each
+            lbm.collide(g, fl)
+            lbm.add_volume_force(g, fl, F)
+            lbm.stream(g, fl)
+        want = fl.get("f").tobytes()
+        fl.set("f", f)
+        lbm.step_single(g, fl, 9, F)
+        assert fl.get("f").tobytes() == want
+        d = sclbm.Domain(nx, ny, mask, sclbm.make_params(ncomp=1, tau=(0.8, 1.0), force=(F, None)), sclbm.FP64)
+        d.upload_f(0, f)
+        d.step(9)
+        assert d.download_f(0).tobytes() == want
