@@ -472,12 +472,16 @@ int sclbm_fluid_compute_f_equilibrium_geom(sclbm_fluid *f, const sclbm_geometry 
     return SCLBM_OK;
 }
 
+static FeqArgs feq_args(const sclbm_fluid *f)
+{
+    return FeqArgs{f->d[SCLBM_FIELD_F],     f->d[SCLBM_FIELD_RHO], f->d[SCLBM_FIELD_UEQ_X],
+                   f->d[SCLBM_FIELD_UEQ_Y], f->d[SCLBM_FIELD_FEQ], f->omega};
+}
+
 int sclbm_fluid_compute_f_equilibrium(sclbm_fluid *f)
 {
     CHECK_NULL(f);
-    CUDA_LAUNCH(op_feq_multi(f->N, f->d[SCLBM_FIELD_F], f->d[SCLBM_FIELD_RHO],
-                             f->d[SCLBM_FIELD_UEQ_X], f->d[SCLBM_FIELD_UEQ_Y],
-                             f->d[SCLBM_FIELD_FEQ], f->omega, 0, stream()));
+    CUDA_LAUNCH(op_feq(f->N, feq_args(f), stream()));
     return SCLBM_OK;
 }
 
@@ -692,10 +696,7 @@ int sclbm_lbm_collide(sclbm_lbm *l, sclbm_fluid *f1, sclbm_fluid *f2)
     CHECK_NULL(f2);
     if (f1->N != l->N || f2->N != l->N)
         return set_error(SCLBM_E_INVALID_ARGUMENT, "LBM and fluid sizes differ");
-    for (sclbm_fluid *f : {f1, f2})
-        CUDA_LAUNCH(op_feq_multi(f->N, f->d[SCLBM_FIELD_F], f->d[SCLBM_FIELD_RHO],
-                                 f->d[SCLBM_FIELD_UEQ_X], f->d[SCLBM_FIELD_UEQ_Y],
-                                 f->d[SCLBM_FIELD_FEQ], f->omega, 1, stream()));
+    CUDA_LAUNCH(op_collide(l->N, feq_args(f1), feq_args(f2), stream()));
     return SCLBM_OK;
 }
 
@@ -713,7 +714,7 @@ int sclbm_lbm_add_volume_force_single(sclbm_lbm *l, const sclbm_geometry *g, scl
     const uint8_t *m;
     int rc = lbm_prep(l, g, f, nullptr, &m);
     if (rc || (rc = check_force(force, count))) return rc;
-    CUDA_LAUNCH(op_volume_force(f->N, m, f->d[SCLBM_FIELD_F], force, stream()));
+    CUDA_LAUNCH(op_volume_force(f->N, m, f->d[SCLBM_FIELD_F], nullptr, force, stream()));
     return SCLBM_OK;
 }
 
@@ -724,8 +725,7 @@ int sclbm_lbm_add_volume_force(sclbm_lbm *l, const sclbm_geometry *g, sclbm_flui
     CHECK_NULL(f2);
     int rc = lbm_prep(l, g, f1, f2, &m);
     if (rc || (rc = check_force(force, count))) return rc;
-    CUDA_LAUNCH(op_volume_force(f1->N, m, f1->d[SCLBM_FIELD_F], force, stream()));
-    CUDA_LAUNCH(op_volume_force(f2->N, m, f2->d[SCLBM_FIELD_F], force, stream()));
+    CUDA_LAUNCH(op_volume_force(f1->N, m, f1->d[SCLBM_FIELD_F], f2->d[SCLBM_FIELD_F], force, stream()));
     return SCLBM_OK;
 }
 
@@ -734,7 +734,8 @@ int sclbm_lbm_stream_single(sclbm_lbm *l, const sclbm_geometry *g, sclbm_fluid *
     const uint8_t *m;
     int rc = lbm_prep(l, g, f, nullptr, &m);
     if (rc) return rc;
-    CUDA_LAUNCH(op_stream((int)g->nx, (int)g->ny, m, f->d[SCLBM_FIELD_F], l->d_tmp[0], stream()));
+    CUDA_LAUNCH(op_stream((int)g->nx, (int)g->ny, m, g->has_solid, f->d[SCLBM_FIELD_F], l->d_tmp[0], nullptr,
+                          nullptr, stream()));
     std::swap(f->d[SCLBM_FIELD_F], l->d_tmp[0]); // std::swap(temp_f_dist, f_dist), src/lbm.cpp:382
     return SCLBM_OK;
 }
@@ -745,8 +746,8 @@ int sclbm_lbm_stream(sclbm_lbm *l, const sclbm_geometry *g, sclbm_fluid *f1, scl
     CHECK_NULL(f2);
     int rc = lbm_prep(l, g, f1, f2, &m);
     if (rc) return rc;
-    CUDA_LAUNCH(op_stream((int)g->nx, (int)g->ny, m, f1->d[SCLBM_FIELD_F], l->d_tmp[0], stream()));
-    CUDA_LAUNCH(op_stream((int)g->nx, (int)g->ny, m, f2->d[SCLBM_FIELD_F], l->d_tmp[1], stream()));
+    CUDA_LAUNCH(op_stream((int)g->nx, (int)g->ny, m, g->has_solid, f1->d[SCLBM_FIELD_F], l->d_tmp[0],
+                          f2->d[SCLBM_FIELD_F], l->d_tmp[1], stream()));
     std::swap(f1->d[SCLBM_FIELD_F], l->d_tmp[0]);
     std::swap(f2->d[SCLBM_FIELD_F], l->d_tmp[1]);
     return SCLBM_OK;
