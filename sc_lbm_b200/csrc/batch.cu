@@ -212,8 +212,8 @@ static int upload_args(sclbm_batch *b, const std::vector<int> &ty, const std::ve
 
 // Units of the two-step kernel: per domain its strips and bands, all of about
 // the rows that two_cost finds best for the batch's units (the caller's height
-// where given).  64 mixed domains: 24 rows 80 us per step, 16 rows 85, 32 rows
-// 98, 64 rows 92 (ring body 104).
+// where given).  64 mixed domains, before the node codes: 24 rows 80 us per
+// step, 16 rows 85, 32 rows 98, 64 rows 92 (ring body 104).
 static int build_two(sclbm_batch *b, const int *tile_y)
 {
     if (b->prec == SCLBM_FP64) return SCLBM_OK;

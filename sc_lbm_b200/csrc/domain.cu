@@ -47,6 +47,38 @@ __global__ void k_upload_dir(size_t N, const uint8_t *__restrict__ mask,
     GRID_STRIDE(n, N) { dst[n] = Conv<S>::from_f64(mask[n] ? src[n] - shift : 0.0); }
 }
 
+// Node codes of a mask and the table of solid sums (CodeMask): what a collision
+// needs to know of the solid nodes around it, in one 2-byte load instead of
+// nine mask bytes, and in one table entry instead of 24 selects and additions
+// (the same additions in the same order).
+__global__ void k_codes(int nx, int ny, const uint8_t *__restrict__ mask, uint16_t *__restrict__ codes,
+                        float2 *__restrict__ sums)
+{
+    if (blockIdx.x == 0) {
+        for (int b = threadIdx.x; b < 256; b += blockDim.x) {
+            float x = 0.f, y = 0.f;
+#pragma unroll
+            for (int i = 1; i < 9; ++i) {
+                const bool fluid = (b >> (i - 1)) & 1;
+                if (cx(i)) x += fluid ? 0.f : float(w_sc(i) * cx(i));
+                if (cy(i)) y += fluid ? 0.f : float(w_sc(i) * cy(i));
+            }
+            sums[b] = make_float2(x, y);
+        }
+    }
+    GRID_STRIDE(n, (size_t)nx * ny)
+    {
+        const int y = (int)(n / nx), x = (int)(n - (size_t)y * nx);
+        uint32_t c = mask[n];
+        if (c) {
+#pragma unroll
+            for (int i = 1; i < 9; ++i)
+                c |= (uint32_t)mask[(size_t)wrap1(y + cy(i), ny) * nx + wrap1(x + cx(i), nx)] << i;
+        }
+        codes[n] = (uint16_t)c;
+    }
+}
+
 // Seeded initial state written on the device: f_i = rho/9 on fluid nodes (the
 // reference initialisers' shape, src/lbm.cpp:11-48, src/fluid.cpp:64-104),
 // rho = rho0 * (1 + amp * (2u - 1)) with u the splitmix64 uniform of
@@ -287,6 +319,8 @@ static void fill2(const sclbm_domain *d, Fused2Args<S, T> &a)
     a.has_solid = d->has_solid ? 1 : 0;
     a.solids_zero = 1; // creation, uploads and initialisers write 0 at solid nodes
     a.status = d->d_status;
+    a.codes = d->d_codes;
+    a.sums = d->d_sums;
 }
 
 template <typename S, typename T>
@@ -438,16 +472,16 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
 }
 
 // Whether the domain's steps run in pairs (fused_two.cuh): the shifted forms
-// beyond 600 k (FP32) or 1.1 M (FP16) nodes, where both buffers outgrow L2;
-// below, one node per thread is faster.  us per step, pairs / one node per
-// thread: FP32 512^2 9.3 / 7.5, 768^2 15.4 / 15.4 (with solid nodes 18.9 /
-// 18.7), 1024^2 22.6 / 31.6; FP16 768^2 17.5 / 14.3, 1024^2 24.6 / 24.0 (29.9 /
-// 28.5), 2048 x 1024 44 / 47.5.  Lattices that need 64-bit offsets, and domains
-// with a variant or a tile width of the caller's choice, take single steps; a
-// band height of the caller's choice asks for pairs.
+// beyond 450 k (FP32) or 1.5 M (FP16) nodes; below, where the buffers fit L2,
+// one node per thread is faster.  us per step, pairs / one node per thread:
+// FP32 600^2 11.3 / 10.0 (with solid nodes 12.4 / 12.3), 700^2 12.3 / 12.9 (14.4
+// / 15.8), 1024^2 22.6 / 31.6; FP16 1024^2 24.6 / 24.0 (27.8 / 26.3), 1200^2 33 /
+// 33 (39 / 37), 2048 x 1024 44 / 47.5 (52 / 52).  Lattices that need 64-bit
+// offsets, and domains with a variant or a tile width of the caller's choice,
+// take single steps; a band height of the caller's choice asks for pairs.
 static bool two_step(const sclbm_domain *d)
 {
-    const size_t most = d->prec == SCLBM_FP32_SHIFTED ? 600000 : 1100000;
+    const size_t most = d->prec == SCLBM_FP32_SHIFTED ? 450000 : 1500000;
     return d->variant == 0 && d->tx == 128 && d->ncomp == 2 && d->prec != SCLBM_FP64 && d->nx >= 4 &&
            d->ny >= 4 && (d->tile_y > 0 || d->N > most) && !needs_wide_offsets(d->N);
 }
@@ -527,6 +561,16 @@ int domain_launch_step(sclbm_domain *d, cudaStream_t s)
 
 using namespace sclbm;
 
+namespace sclbm {
+int domain_refresh_codes(sclbm_domain *d, cudaStream_t s)
+{
+    if (!d->d_codes) return SCLBM_OK;
+    k_codes<<<grid_for(d->N, 256), 256, 0, s>>>((int)d->nx, (int)d->ny, d->d_mask, d->d_codes, d->d_sums);
+    SCLBM_LAUNCHED("node codes");
+    return SCLBM_OK;
+}
+} // namespace sclbm
+
 static int dom_alloc(sclbm_domain *d, void **p, size_t bytes)
 {
     cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
@@ -547,6 +591,7 @@ void sclbm_domain_destroy(sclbm_domain *d)
     for (auto *p : d->rho_tmp)
         if (p) cudaFree(p);
     if (d->d_mask) cudaFree(d->d_mask);
+    if (d->d_codes) cudaFree(d->d_codes);
     if (d->staging) cudaFree(d->staging);
     if (d->partials) cudaFree(d->partials);
     if (d->d_status) cudaFree(d->d_status);
@@ -605,8 +650,13 @@ int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_p
         rc = set_error(SCLBM_E_CUDA, "memset");
         goto fail;
     }
+    if (precision != SCLBM_FP64 && d->ncomp == 2) {
+        const size_t codes = (N * sizeof(uint16_t) + 15) & ~size_t(15);
+        if ((rc = dom_alloc(d, (void **)&d->d_codes, codes + 256 * sizeof(float2)))) goto fail;
+        d->d_sums = (float2 *)((char *)d->d_codes + codes);
+    }
     if (cudaMemcpyAsync(d->d_mask, hm.data(), N, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess) {
+        domain_refresh_codes(d, s) != SCLBM_OK || cudaStreamSynchronize(s) != cudaSuccess) {
         rc = set_error(SCLBM_E_CUDA, "mask upload");
         goto fail;
     }

@@ -8,6 +8,8 @@ struct sclbm_domain {
     sclbm_precision prec = SCLBM_FP64;
     sclbm_params p{};
     uint8_t *d_mask = nullptr;
+    uint16_t *d_codes = nullptr; // node codes of the mask (two-component shifted forms), and
+    float2 *d_sums = nullptr;    // behind them the sums by neighbour bits
     void *buf[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}; // [parity][comp], 9N each
     int parity = 0; // buf[parity] holds the state; turns over with every step
     void *rho_tmp[2] = {nullptr, nullptr}; // density arrays of the two-pass variant
@@ -26,6 +28,7 @@ struct sclbm_domain {
 namespace sclbm {
 size_t elem_size(sclbm_precision p);
 int domain_launch_step(sclbm_domain *d, cudaStream_t s);
+int domain_refresh_codes(sclbm_domain *d, cudaStream_t s); // after the device mask has changed
 int domain_default_tile_y(const sclbm_domain *d);
 int domain_field_async(sclbm_domain *d, int comp, int what, double *host, cudaStream_t s);
 // fill the kernel argument blocks for the current parity

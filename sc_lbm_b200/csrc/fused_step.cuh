@@ -215,6 +215,37 @@ template <typename T> struct Stencil {
     int c;
 };
 
+// Where a node's neighbour flags come from.  MaskStencil reads the mask rows of
+// the density stencil; CodeMask reads one node code (Fused2Args::codes): bit 0
+// the node, bit i its neighbour along c_i, 1 for fluid, the neighbours' bits
+// cleared at solid nodes (the uniform solid form).  nf(i) is 0 or 1; sums adds
+// up w c_i over the solid neighbours (src/lbm.cpp:131-134).
+template <typename T, bool UNIFORM> struct MaskStencil {
+    const Stencil<T> &st;
+    __device__ __forceinline__ uint32_t self() const { return st.m[1][st.c]; }
+    __device__ __forceinline__ uint32_t nf(int i) const
+    {
+        return (uint32_t)st.m[cy(i) + 1][st.c + cx(i)] & (UNIFORM ? self() : 1u);
+    }
+    __device__ __forceinline__ float2 sums(const uint32_t (&n)[9]) const
+    {
+        float x = 0.f, y = 0.f;
+#pragma unroll
+        for (int i = 1; i < 9; ++i) {
+            if (cx(i)) x += n[i] ? 0.f : float(w_sc(i) * cx(i));
+            if (cy(i)) y += n[i] ? 0.f : float(w_sc(i) * cy(i));
+        }
+        return make_float2(x, y);
+    }
+};
+struct CodeMask {
+    uint32_t code;
+    const float2 *table; // sums by neighbour bits (Fused2Args::sums)
+    __device__ __forceinline__ uint32_t self() const { return code & 1u; }
+    __device__ __forceinline__ uint32_t nf(int i) const { return (code << (31 - i)) >> 31; }
+    __device__ __forceinline__ float2 sums(const uint32_t (&)[9]) const { return table[code >> 1]; }
+};
+
 // 32-bit indices of a node (nb[0]) and of its periodic neighbours along c_i
 struct Nbr {
     uint32_t nb[9];
@@ -283,6 +314,7 @@ __device__ __forceinline__ void push_one_raw(const Fused2Args<S, T> &a, const in
 // of a solid node (solid); node() is the lattice index of the node.
 // This one pushes into the output arrays of the launch.
 template <typename S, typename T, bool SOLID, bool WIDE> struct GlobalSink {
+    static constexpr bool SOLID_ZEROS = true; // solid lanes of the uniform form hand over zeros
     const Fused2Args<S, T> &a;
     const Nbr &n;
     __device__ __forceinline__ uint32_t node() const { return n.nb[0]; }
@@ -318,16 +350,17 @@ template <typename S, typename T, bool SOLID, bool WIDE> struct GlobalSink {
 // sequence of src/lbm.cpp:177-204 (repulsive force), :250-269 (equilibrium
 // velocity), src/fluid.cpp:254-276 + src/lbm.cpp:305-311 (equilibrium, BGK),
 // :333-337 (volume force), :404-427 (stream with half-way bounce-back).
-template <typename S, typename T, int FLAGS, typename Pops, typename Sink>
+template <typename S, typename T, int FLAGS, typename Pops, typename Sink, typename Mask>
 __device__ __forceinline__ void collide_node(const Fused2Args<S, T> &a, const Pops &f,
-                                             const Stencil<T> &st, const Sink &sink)
+                                             const Stencil<T> &st, const Sink &sink, const Mask &mask)
 {
     constexpr bool EXACT = sizeof(T) == 8;
     constexpr bool FORCE = (FLAGS & KF_FORCE) != 0, SOLID = (FLAGS & KF_SOLID) != 0;
     constexpr bool UNIFORM = SOLID && (FLAGS & KF_UNIFORM) != 0;
+    constexpr bool ZEROS = UNIFORM && Sink::SOLID_ZEROS;
     // a solid lane of the uniform form treats every neighbour as solid: its
     // nine stores then land in its own slots, and carry zeros
-    const bool self_fluid = !SOLID || st.m[1][st.c] != 0;
+    const bool self_fluid = !SOLID || mask.self() != 0;
     if (SOLID && !UNIFORM && !self_fluid) {
         sink.solid();
         return;
@@ -335,12 +368,11 @@ __device__ __forceinline__ void collide_node(const Fused2Args<S, T> &a, const Po
     // nf[i] = 1 when the neighbour along c_i is a fluid node (mask bytes are 0 or 1)
     uint32_t nf[9];
     T p0[9], p1[9];
-    const uint32_t self_u = SOLID ? (uint32_t)st.m[1][st.c] : 1u;
 #pragma unroll
     for (int i = 1; i < 9; ++i) {
         const int sl = cy(i) + 1;
         const int col = st.c + cx(i);
-        nf[i] = SOLID ? (uint32_t)st.m[sl][col] & (UNIFORM ? self_u : 1u) : 1u;
+        nf[i] = SOLID ? mask.nf(i) : 1u;
         const V2<T> v = st.r[sl][col];
         p0[i] = v.x;
         p1[i] = v.y;
@@ -421,17 +453,15 @@ __device__ __forceinline__ void collide_node(const Fused2Args<S, T> &a, const Po
         const PairParams<T> &pc = a.pc;
         // Ps.x = sum_i w c_i drho_0(nbr), Ps.y = sum_i w c_i drho_1(nbr)
         float2 Psx = f2(0.f), Psy = f2(0.f);
-        float Sx = 0.f, Sy = 0.f;
+        float2 S2 = f2(0.f);
+        if constexpr (SOLID) S2 = mask.sums(nf);
+        const float Sx = S2.x, Sy = S2.y;
 #pragma unroll
         for (int i = 1; i < 9; ++i) {
             const float wcx = float(w_sc(i) * cx(i)), wcy = float(w_sc(i) * cy(i));
             const float2 q = make_float2(p0[i], p1[i]);
             if (cx(i)) Psx = fma2(f2(wcx), q, Psx);
             if (cy(i)) Psy = fma2(f2(wcy), q, Psy);
-            if constexpr (SOLID) {
-                if (cx(i)) Sx += nf[i] ? 0.f : wcx;
-                if (cy(i)) Sy += nf[i] ? 0.f : wcy;
-            }
         }
         const float2 RR = pair_of(pc.rho_ref);
         const float2 DR = make_float2(psi0, psi1);
@@ -491,7 +521,7 @@ __device__ __forceinline__ void collide_node(const Fused2Args<S, T> &a, const Po
                 // mass with the rounded values
                 const __half2 H = __float22half2_rn(V);
                 __half h0 = __low2half(H), h1 = __high2half(H);
-                if constexpr (UNIFORM) {
+                if constexpr (ZEROS) {
                     h0 = self_fluid ? h0 : __float2half_rn(0.f);
                     h1 = self_fluid ? h1 : __float2half_rn(0.f);
                 }
@@ -499,7 +529,7 @@ __device__ __forceinline__ void collide_node(const Fused2Args<S, T> &a, const Po
                 return sub2(fp(i), __half22float2(H));
             } else {
                 float v0 = V.x, v1 = V.y;
-                if constexpr (UNIFORM) {
+                if constexpr (ZEROS) {
                     v0 = self_fluid ? v0 : 0.f;
                     v1 = self_fluid ? v1 : 0.f;
                 }
@@ -526,13 +556,13 @@ __device__ __forceinline__ void collide_node(const Fused2Args<S, T> &a, const Po
         if constexpr (sizeof(S) == 2) {
             const __half2 H = __float22half2_rn(V0);
             __half h0 = __low2half(H), h1 = __high2half(H);
-            if constexpr (UNIFORM) {
+            if constexpr (ZEROS) {
                 h0 = self_fluid ? h0 : __float2half_rn(0.f);
                 h1 = self_fluid ? h1 : __float2half_rn(0.f);
             }
             sink.pair_half(0, h0, h1, nf[0]);
         } else {
-            if constexpr (UNIFORM) {
+            if constexpr (ZEROS) {
                 V0.x = self_fluid ? V0.x : 0.f;
                 V0.y = self_fluid ? V0.y : 0.f;
             }
@@ -547,7 +577,8 @@ template <typename S, typename T, int FLAGS, bool WIDE = false, typename Pops>
 __device__ __forceinline__ void collide_push(const Fused2Args<S, T> &a, const Pops &f,
                                              const Stencil<T> &st, const Nbr &n)
 {
-    collide_node<S, T, FLAGS>(a, f, st, GlobalSink<S, T, (FLAGS & KF_SOLID) != 0, WIDE>{a, n});
+    collide_node<S, T, FLAGS>(a, f, st, GlobalSink<S, T, (FLAGS & KF_SOLID) != 0, WIDE>{a, n},
+                              MaskStencil<T, (FLAGS & KF_UNIFORM) != 0>{st});
 }
 
 // shared-memory view of one node's populations in a ring: f[k][i]

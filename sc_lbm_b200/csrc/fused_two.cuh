@@ -7,9 +7,11 @@
 // steps lives in shared memory, a few rows at a time.  What bounds it then is
 // the FP32 pipe (packed instructions: 58 % busy) and, over seconds, the
 // board's power limit; DRAM is half busy.  Measured on one B200, us per step
-// (the one-step ring kernel before): FP32 4096^2 270 (407), its 60 % fluid
-// form 337 (459), FP16 4096^2 277 (334), FP32 1024^2 22.6 (35.5), 256^2 5.4
-// (8.2).  FP64 stays with the one-step kernels: its rows between the steps
+// (the one-step kernels before): FP32 4096^2 267 (407), its 60 % fluid form 327
+// (459), FP16 4096^2 277 (334) and 351 (442), FP32 2048 x 1024 with 40 % solid
+// nodes 46 (78), 1024^2 22.6 (35.5).  With solid nodes a node step took 469
+// instructions against 309; node codes in place of mask bytes and sums (and no
+// zeros between the steps) gave 2 to 9 % there.  FP64 stays with the one-step kernels: its rows between the steps
 // leave two CTAs per SM, and 12 % busy warps ran no faster (398 against 388
 // on 4096 x 2048, 546 against 485 with solid nodes).
 //
@@ -67,7 +69,7 @@ template <typename S, int TX> struct __align__(16) TwoShared {
     static constexpr int LEVEL = 3 * ROW, BEHIND = 5 * ROW;
     typename TwoCell<S>::type m[7 * ROW];
     float2 rho1[3][TX], rho2[3][TX]; // densities before the first and second step
-    uint8_t msk[8][TX];              // mask rows q-7 .. q
+    uint16_t code[8][TX];            // node codes of the rows q-7 .. q, each read by its own thread
 };
 
 // place of direction i among the three of its class (opposite ones alike)
@@ -86,6 +88,7 @@ struct TwoRow {
 // pushes a first-step node's populations into the rows between the steps;
 // to: the destination rows of the three classes, own: the node's own row
 template <typename S, int TX, bool SOLID> struct SharedSink {
+    static constexpr bool SOLID_ZEROS = false; // solid nodes' slots are never used
     typename TwoCell<S>::type *m;
     TwoRow to, own;
     __device__ __forceinline__ int slot(int i, uint32_t nf) const
@@ -143,7 +146,7 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
     const int xl = wrap1(x - 1, nx), xr = wrap1(x + 1, nx);
     auto gy = [&](int q) { return wrap3(y0 + (down ? nrow - 1 - q : q), ny); };
 
-    uint8_t mask_ahead = 1;
+    uint16_t code_ahead = 0x1ff;
     // all-fluid lattices load on every thread (idle ones column 0): without the
     // branch the loads of FP16 rows sit earlier (4096^2: 309 -> 289 us a step,
     // FP32 286 -> 280); with solid nodes the branch was the faster form (337
@@ -151,7 +154,7 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
     auto load_row = [&](int q, float(&f)[2][9]) {
         if (SOLID && !load) return;
         const uint32_t node = (uint32_t)gy(q) * (uint32_t)nx + (uint32_t)x;
-        if (SOLID) mask_ahead = a.mask[node];
+        if (SOLID) code_ahead = a.codes[node];
 #pragma unroll
         for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -177,7 +180,8 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
         const int ahead = s * L::ROW + t, two = (r & 1) * L::ROW + t;
         return TwoRow{down ? ahead : L::BEHIND + two, L::LEVEL + two, down ? L::BEHIND + two : ahead};
     };
-    auto mrow = [&](int p) { return (const uint8_t *)sh.msk[(p + 8) & 7]; };
+    // mask of this thread's node in row r (without solid nodes not used)
+    auto code_of = [&](int r) { return SOLID ? (uint32_t)sh.code[(r + 8) & 7][t] : 0x1ffu; };
 
     // cur: row q, prev: row q - 1, both before step 1; mcur: row q - 3, mprev:
     // row q - 4, both after it
@@ -187,39 +191,39 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
             float r0, r1;
             two_read<S, TX>(sh, row_at(s0, q - 3), mcur);
             node_density(mcur, r0, r1);
-            if (SOLID && !mrow(q - 3)[t]) r0 = r1 = 0.f;
+            if (SOLID && !(code_of(q - 3) & 1u)) r0 = r1 = 0.f;
             sh.rho2[s0][t] = make_float2(r0, r1);
         }
         if (load && q <= nrow + 2) {
             float r0, r1;
             node_density(cur, r0, r1);
             if (SOLID) {
-                if (!mask_ahead) r0 = r1 = 0.f;
-                sh.msk[(q + 8) & 7][t] = mask_ahead;
+                if (!(code_ahead & 1u)) r0 = r1 = 0.f;
+                sh.code[(q + 8) & 7][t] = code_ahead;
             }
             sh.rho1[s0][t] = make_float2(r0, r1);
         }
         __syncthreads();
         const int lo = down ? s0 : s2, hi = down ? s2 : s0; // rows below and above the node
         if (step1 && q >= -1 && q <= nrow + 2) {
-            const Stencil<float> st{{sh.rho1[lo], sh.rho1[s1], sh.rho1[hi]},
-                                    {mrow(down ? q : q - 2), mrow(q - 1), mrow(down ? q - 2 : q)}, t};
+            const Stencil<float> st{{sh.rho1[lo], sh.rho1[s1], sh.rho1[hi]}, {}, t};
             // ahead: row q; level: row q - 1; behind: row q - 2
             const TwoRow own = row_at(s1, q - 1);
             const int ahead = s0 * L::ROW + t, behind = L::BEHIND + (q & 1) * L::ROW + t;
             const TwoRow to{down ? ahead : behind, own.level, down ? behind : ahead};
-            collide_node<S, float, FLAGS>(a, prev, st, SharedSink<S, TX, SOLID>{sh.m, to, own});
+            collide_node<S, float, FLAGS>(a, prev, st, SharedSink<S, TX, SOLID>{sh.m, to, own},
+                                          CodeMask{code_of(q - 1), a.sums});
         }
         if (!SOLID) load_row(min(q + 1, nrow + 2), prev);
         else if (q < nrow + 2) load_row(q + 1, prev);
         if (!SOLID && pf != nullptr && q + 2 <= nrow + 2)
             asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + (size_t)gy(q + 2) * (size_t)nx));
         if (step2 && q >= 4 && q <= nrow + 3) {
-            const Stencil<float> st{{sh.rho2[lo], sh.rho2[s1], sh.rho2[hi]},
-                                    {mrow(down ? q - 3 : q - 5), mrow(q - 4), mrow(down ? q - 5 : q - 3)}, t};
+            const Stencil<float> st{{sh.rho2[lo], sh.rho2[s1], sh.rho2[hi]}, {}, t};
             const int yc = gy(q - 4);
             const Nbr n = make_nbr(nx, x, xl, xr, yc, wrap1(yc - 1, ny), wrap1(yc + 1, ny));
-            collide_push<S, float, FLAGS>(a, mprev, st, n);
+            collide_node<S, float, FLAGS>(a, mprev, st, GlobalSink<S, float, SOLID, false>{a, n},
+                                          CodeMask{code_of(q - 4), a.sums});
         }
         __syncthreads();
         const int s = s2;
@@ -287,10 +291,10 @@ inline int two_width(int nx)
 // last, partial wave an iteration with n CTAs on an SM takes longer than n
 // shares, down to the latency of one (measured with solid nodes, where a share
 // is 0.66 us: 1.6, 1.9, 2.45 and 2.9 us for one to four).  Measured by this
-// choice / other heights, us per step: 1021 x 763 12 rows 21.9 / 8 rows 25.0,
-// 24 rows 23.6; 1024^2 16 rows 22.6 / 12 rows 26.0, 24 rows 24.7; 256^2 3 rows
-// 5.4 / 6 rows 6.2; a batch of eight 400 x 306 20 rows 35.9 / 16 rows 49.5, 6
-// rows 39.3; 4096^2 within 2 % from 48 to 96 rows.
+// choice / other heights, us per step: 1021 x 763 12 rows 20.5 / 16 rows 21.4;
+// 1024^2 16 rows 22.6 / 12 rows 26.0, 24 rows 24.7; 2048 x 1024 32 rows 47.3 / 40
+// rows 48.2; a batch of eight 400 x 306 20 rows 32.9 / 24 rows 34.1; 4096^2
+// within 2 % from 48 to 96 rows.
 constexpr int TWO_ROWS[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64};
 inline double two_cost(long units, int r, int sms)
 {

@@ -125,6 +125,9 @@ template <typename S, typename T> struct Fused2Args {
     int has_solid;                       // the mask has solid nodes (else all fluid)
     int solids_zero;                     // both buffers hold 0 at solid nodes: the kernels
                                          // neither read nor write them (domain path)
+    const uint16_t *codes;               // float arithmetic: per node its own and its neighbours'
+                                         // fluid bits (CodeMask in fused_step.cuh)
+    const float2 *sums;                  // sum of w c_i over solid neighbours by neighbour bits
     int *status;                         // set to 1 by a kernel whose bounded wait ran out
                                          // (ring kernel), or null
     int row0, row_end;                   // register tile: step the rows [row0, row_end)

@@ -297,6 +297,8 @@ extern "C" int sclbm_domain_add_random_disks(sclbm_domain *d, double porosity, i
         }
         SCLBM_LAUNCHED("packing: rasterisation");
         d->has_solid = true;
+        const int rc = domain_refresh_codes(d, s);
+        if (rc) return rc;
     }
     SCLBM_CUDA(cudaStreamSynchronize(s));
     if (placed) *placed = ndisks;

@@ -39,7 +39,7 @@ def state(d):
 
 @pytest.mark.parametrize("prec_name", ["FP32_SHIFTED", "FP16_SHIFTED"])
 @pytest.mark.parametrize("nx,ny,rows", [(4, 4, 2), (5, 7, 1), (64, 33, 5), (121, 20, 20), (122, 9, 4),
-                                        (123, 40, 32), (245, 31, 3), (1021, 77, 7), (1200, 1000, 0)])
+                                        (123, 40, 32), (245, 31, 3), (1021, 77, 7), (1400, 1100, 0)])
 def test_pairs_match_single_steps(sclbm, prec_name, nx, ny, rows):
     prec = getattr(sclbm, prec_name)
     for porous in (False, True):
