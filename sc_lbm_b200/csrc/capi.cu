@@ -359,6 +359,7 @@ int sclbm_fluid_create(size_t nx, size_t ny, double tau, sclbm_fluid **out)
     if (rc) return rc;
     auto *f = new (std::nothrow) sclbm_fluid();
     if (!f) return set_error(SCLBM_E_ALLOC, "host allocation failed");
+    host_copy_retain();
     f->nx = nx;
     f->ny = ny;
     f->N = nx * ny;
@@ -383,6 +384,7 @@ void sclbm_fluid_destroy(sclbm_fluid *f)
     for (auto *p : f->d)
         if (p) cudaFree(p);
     delete f;
+    host_copy_release();
 }
 
 int sclbm_fluid_set_interactions(sclbm_fluid *f, double g_solid, double g_fluid)
@@ -423,9 +425,7 @@ int sclbm_fluid_read(sclbm_fluid *f, sclbm_field field, double *dst, size_t coun
     if (count != field_count(f, field))
         return set_error(SCLBM_E_INVALID_ARGUMENT, "field size mismatch");
     if (count && !dst) return set_error(SCLBM_E_INVALID_ARGUMENT, "null destination");
-    SCLBM_CUDA(cudaMemcpyAsync(dst, f->d[field], count * sizeof(double), cudaMemcpyDeviceToHost,
-                               stream()));
-    SCLBM_CUDA(cudaStreamSynchronize(stream()));
+    SCLBM_CUDA(copy_to_host(dst, f->d[field], count * sizeof(double), stream()));
     return SCLBM_OK;
 }
 

@@ -596,6 +596,7 @@ void sclbm_domain_destroy(sclbm_domain *d)
     if (d->partials) cudaFree(d->partials);
     if (d->d_status) cudaFree(d->d_status);
     delete d;
+    host_copy_release();
 }
 
 int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_params *p,
@@ -622,6 +623,7 @@ int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_p
     }
     auto *d = new (std::nothrow) sclbm_domain();
     if (!d) return set_error(SCLBM_E_ALLOC, "host allocation failed");
+    host_copy_retain();
     d->nx = nx;
     d->ny = ny;
     d->N = N;
@@ -818,9 +820,10 @@ int sclbm_domain_download_f(sclbm_domain *d, int comp, double *f, size_t count)
     cudaStream_t s = stream();
     const void *src = d->buf[d->parity][comp];
     if (d->prec == SCLBM_FP64) {
-        SCLBM_CUDA(cudaMemcpyAsync(f, src, 9 * d->N * 8, cudaMemcpyDeviceToHost, s));
+        SCLBM_CUDA(copy_to_host(f, src, 9 * d->N * 8, s));
     } else {
         const double rr = d->p.rho_ref[comp];
+        const bool bounced = host_copy_bounced(f, d->N * 8);
         for (int i = 0; i < 9; ++i) {
             if (d->prec == SCLBM_FP32_SHIFTED)
                 k_download_dir<float><<<grid_for(d->N, 256), 256, 0, s>>>(
@@ -829,10 +832,12 @@ int sclbm_domain_download_f(sclbm_domain *d, int comp, double *f, size_t count)
                 k_download_dir<__half><<<grid_for(d->N, 256), 256, 0, s>>>(
                     d->N, d->d_mask, (const __half *)src + i * d->N, d->staging, w_eq(i) * rr);
             SCLBM_LAUNCHED("download conversion");
-            SCLBM_CUDA(cudaMemcpyAsync(f + i * d->N, d->staging, d->N * 8, cudaMemcpyDeviceToHost, s));
+            if (bounced) SCLBM_CUDA(copy_to_host(f + i * d->N, d->staging, d->N * 8, s));
+            else
+                SCLBM_CUDA(cudaMemcpyAsync(f + i * d->N, d->staging, d->N * 8, cudaMemcpyDeviceToHost, s));
         }
+        SCLBM_CUDA(cudaStreamSynchronize(s));
     }
-    SCLBM_CUDA(cudaStreamSynchronize(s));
     return SCLBM_OK;
 }
 
@@ -911,8 +916,7 @@ int sclbm_domain_download_rho(sclbm_domain *d, int comp, double *rho, size_t cou
     if (!rho) return set_error(SCLBM_E_INVALID_ARGUMENT, "null rho");
     cudaStream_t s = stream();
     if ((rc = rho_to_staging(d, comp, s))) return rc;
-    SCLBM_CUDA(cudaMemcpyAsync(rho, d->staging, d->N * 8, cudaMemcpyDeviceToHost, s));
-    SCLBM_CUDA(cudaStreamSynchronize(s));
+    SCLBM_CUDA(copy_to_host(rho, d->staging, d->N * 8, s));
     return SCLBM_OK;
 }
 
@@ -932,6 +936,11 @@ int sclbm_domain_download_velocity(sclbm_domain *d, int comp, double *ux, double
     default: k_velocity<__half><<<g, 256, 0, s>>>(d->N, d->d_mask, (const __half *)src, a, b, rr, 1); break;
     }
     SCLBM_LAUNCHED("velocity");
+    if (host_copy_bounced(ux, d->N * 8)) {
+        SCLBM_CUDA(copy_to_host(ux, a, d->N * 8, s));
+        SCLBM_CUDA(copy_to_host(uy, b, d->N * 8, s));
+        return SCLBM_OK;
+    }
     SCLBM_CUDA(cudaMemcpyAsync(ux, a, d->N * 8, cudaMemcpyDeviceToHost, s));
     SCLBM_CUDA(cudaMemcpyAsync(uy, b, d->N * 8, cudaMemcpyDeviceToHost, s));
     SCLBM_CUDA(cudaStreamSynchronize(s));
