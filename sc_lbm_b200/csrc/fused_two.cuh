@@ -7,11 +7,11 @@
 // steps lives in shared memory, a few rows at a time.  What bounds it then is
 // the FP32 pipe (packed instructions: 58 % busy) and, over seconds, the
 // board's power limit; DRAM is half busy.  Measured on one B200, us per step
-// (the one-step kernels before): FP32 4096^2 267 (407), its 60 % fluid form 327
-// (459), FP16 4096^2 277 (334) and 351 (442), FP32 2048 x 1024 with 40 % solid
+// (the one-step kernels before): FP32 4096^2 267 (407), its 60 % fluid form 322
+// (459), FP16 4096^2 277 (334) and 324 (442), FP32 2048 x 1024 with 40 % solid
 // nodes 46 (78), 1024^2 22.6 (35.5).  With solid nodes a node step took 469
 // instructions against 309; node codes in place of mask bytes and sums (and no
-// zeros between the steps) gave 2 to 9 % there.  FP64 stays with the one-step kernels: its rows between the steps
+// zeros between the steps) gave 4 to 12 % there.  FP64 stays with the one-step kernels: its rows between the steps
 // leave two CTAs per SM, and 12 % busy warps ran no faster (398 against 388
 // on 4096 x 2048, 546 against 485 with solid nodes).
 //
@@ -63,13 +63,14 @@ template <> struct TwoCell<__half> {
 // three, two and two rows of three directions each hold them.  Every slot has
 // one writer; slots of columns and rows that only feed the halo are never
 // read, and a solid node's slots never matter: densities and stencils are
-// masked.  28.7 KB for FP32: 113 KB of an SM stay with its L1 beside four CTAs.
+// masked.  31 KB for FP32: 100 KB of an SM stay with its L1 beside four CTAs.
 template <typename S, int TX> struct __align__(16) TwoShared {
     static constexpr int ROW = 3 * TX; // three directions of a row
     static constexpr int LEVEL = 3 * ROW, BEHIND = 5 * ROW;
     typename TwoCell<S>::type m[7 * ROW];
     float2 rho1[3][TX], rho2[3][TX]; // densities before the first and second step
     uint16_t code[8][TX];            // node codes of the rows q-7 .. q, each read by its own thread
+    float2 sums[256];                // Fused2Args::sums (read from L1 it cost 5 %: the rows stream through)
 };
 
 // place of direction i among the three of its class (opposite ones alike)
@@ -147,12 +148,13 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
     auto gy = [&](int q) { return wrap3(y0 + (down ? nrow - 1 - q : q), ny); };
 
     uint16_t code_ahead = 0x1ff;
-    // all-fluid lattices load on every thread (idle ones column 0): without the
-    // branch the loads of FP16 rows sit earlier (4096^2: 309 -> 289 us a step,
-    // FP32 286 -> 280); with solid nodes the branch was the faster form (337
-    // against 349)
+    // loads on every thread (idle ones column 0), without a branch around them:
+    // the loads of a row sit earlier.  us per step with / without: FP16 4096^2
+    // 289 / 309, with solid nodes 324 / 328; FP32 280 / 286, but with solid nodes
+    // 343 / 320, the form in which the compiler keeps the branch
+    constexpr bool EVERY = !SOLID || sizeof(S) == 2;
     auto load_row = [&](int q, float(&f)[2][9]) {
-        if (SOLID && !load) return;
+        if (!EVERY && !load) return;
         const uint32_t node = (uint32_t)gy(q) * (uint32_t)nx + (uint32_t)x;
         if (SOLID) code_ahead = a.codes[node];
 #pragma unroll
@@ -160,12 +162,12 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
 #pragma unroll
             for (int i = 0; i < 9; ++i) f[k][i] = Store<S>::ld(a.fin[k] + elem<false>(i, a.N, node));
     };
-    // all-fluid lattices ask L2 for the row after the one being loaded, one
-    // 128-byte line per thread (FP16 289 -> 277 us a step, FP32 1-2 %; with
-    // solid nodes within noise)
+    // L2 is asked for the row after the one being loaded, one 128-byte line per
+    // thread (FP16 289 -> 277 us a step, with solid nodes 343 -> 328; FP32 1-2 %; a
+    // batch of 64 mixed domains 73 -> 69)
     constexpr int LINES = (TX * (int)sizeof(S) + 127) / 128 + 1; // lines a row segment touches
     const S *pf = nullptr;
-    if (!SOLID && t < 18 * LINES) {
+    if (t < 18 * LINES) {
         const int arr = t / LINES, l = t % LINES;
         const int col = min(max(xb - 3, 0) + l * (128 / (int)sizeof(S)), nx - 1);
         pf = a.fin[arr >= 9 ? 1 : 0] + (size_t)(arr % 9) * a.N + col;
@@ -212,18 +214,18 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
             const int ahead = s0 * L::ROW + t, behind = L::BEHIND + (q & 1) * L::ROW + t;
             const TwoRow to{down ? ahead : behind, own.level, down ? behind : ahead};
             collide_node<S, float, FLAGS>(a, prev, st, SharedSink<S, TX, SOLID>{sh.m, to, own},
-                                          CodeMask{code_of(q - 1), a.sums});
+                                          CodeMask{code_of(q - 1), sh.sums});
         }
-        if (!SOLID) load_row(min(q + 1, nrow + 2), prev);
+        if (EVERY) load_row(min(q + 1, nrow + 2), prev);
         else if (q < nrow + 2) load_row(q + 1, prev);
-        if (!SOLID && pf != nullptr && q + 2 <= nrow + 2)
+        if (pf != nullptr && q + 2 <= nrow + 2)
             asm volatile("prefetch.global.L2 [%0];" ::"l"(pf + (size_t)gy(q + 2) * (size_t)nx));
         if (step2 && q >= 4 && q <= nrow + 3) {
             const Stencil<float> st{{sh.rho2[lo], sh.rho2[s1], sh.rho2[hi]}, {}, t};
             const int yc = gy(q - 4);
             const Nbr n = make_nbr(nx, x, xl, xr, yc, wrap1(yc - 1, ny), wrap1(yc + 1, ny));
             collide_node<S, float, FLAGS>(a, mprev, st, GlobalSink<S, float, SOLID, false>{a, n},
-                                          CodeMask{code_of(q - 4), a.sums});
+                                          CodeMask{code_of(q - 4), sh.sums});
         }
         __syncthreads();
         const int s = s2;
@@ -232,6 +234,8 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
         s0 = s;
     };
 
+    if (SOLID) // read after the first barrier
+        for (int i = t; i < 256; i += TX) sh.sums[i] = a.sums[i];
     float A[2][9], B[2][9], C[2][9], D[2][9];
 #pragma unroll
     for (int k = 0; k < 2; ++k)
