@@ -29,14 +29,19 @@ namespace sclbm {
 
 constexpr int FLAT_ROWS = 4;
 
+// a tile of a batch's list: columns from x0, rows from y0 of domain dom
+struct FlatTile {
+    int dom, x0, y0;
+};
+
 // Resident CTAs per SM the register cap aims at: six for float arithmetic (80
 // registers; five ran 2-5 % slower with solid nodes), four for FP64 (its
 // solid forms take 108 registers; capped at 96 for five they ran 8-25 % slower)
 template <typename T> constexpr int flat_ctas() { return sizeof(T) == 8 ? 4 : 6; }
 
+// One step of the tile [x0, x0 + 32) x [y0, y0 + TY) of a's lattice.
 template <typename S, typename T, int TY, int FLAGS>
-__global__ void __launch_bounds__(32 * TY, (flat_ctas<T>()))
-    k_flat2(const __grid_constant__ Fused2Args<S, T> a)
+__device__ __forceinline__ void flat_tile(const Fused2Args<S, T> &a, const int x0, const int y0)
 {
     constexpr bool SOLID = (FLAGS & KF_SOLID) != 0;
     constexpr int C = 34, HALO = 2 * C + 2 * TY;
@@ -44,7 +49,6 @@ __global__ void __launch_bounds__(32 * TY, (flat_ctas<T>()))
     __shared__ V2<T> rho[TY + 2][C];
     __shared__ uint8_t msk[TY + 2][C];
     const int t = threadIdx.x, nx = a.nx, ny = a.ny;
-    const int x0 = blockIdx.x * 32, y0 = blockIdx.y * TY;
     const int ncol = min(32, nx - x0), nrow = min(TY, ny - y0);
     // this thread's node: column c, row r of the tile with its halo
     const int c = (t & 31) + 1, r = t / 32 + 1;
@@ -107,6 +111,30 @@ __global__ void __launch_bounds__(32 * TY, (flat_ctas<T>()))
         collide_push<S, T, FLAGS>(a, f, st, n);
 }
 
+template <typename S, typename T, int TY, int FLAGS>
+__global__ void __launch_bounds__(32 * TY, (flat_ctas<T>()))
+    k_flat2(const __grid_constant__ Fused2Args<S, T> a)
+{
+    flat_tile<S, T, TY, FLAGS>(a, blockIdx.x * 32, blockIdx.y * TY);
+}
+
+// A batch: CTA b takes tile b of the list.  doms holds two entries per domain
+// (buffer parity 0 and 1); the tile's argument block, which no step writes, is
+// copied into shared memory while the step before ends.
+template <typename S, typename T, int TY, int FLAGS>
+__global__ void __launch_bounds__(32 * TY, (flat_ctas<T>()))
+    k_batch_flat(const Fused2Args<S, T> *__restrict__ doms, const FlatTile *__restrict__ tiles, int parity)
+{
+    __shared__ __align__(16) Fused2Args<S, T> sa;
+    static_assert(sizeof(sa) % 4 == 0, "argument block copied as words");
+    const FlatTile u = tiles[blockIdx.x];
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(doms + 2 * u.dom + parity);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(&sa);
+    for (int w = threadIdx.x; w < (int)(sizeof(sa) / 4); w += 32 * TY) dst[w] = src[w];
+    __syncthreads();
+    flat_tile<S, T, TY, FLAGS>(sa, u.x0, u.y0);
+}
+
 // UNI: lattices with solid nodes run the uniform solid form (FP32/FP16; FP64
 // ran 15 % slower in it on 520 x 260 and 1.5 % faster from 1024^2)
 template <typename S, typename T, int UNI>
@@ -121,6 +149,22 @@ inline cudaError_t launch_flat2_any(const Fused2Args<S, T> &a, cudaStream_t s)
     case KF_SOLID: return launch_dependent(k_flat2<S, T, TY, KF_SOLID | UNI>, grid, block, 0, s, a);
     default: return launch_dependent(k_flat2<S, T, TY, KF_FORCE | KF_SOLID | UNI>, grid, block, 0, s, a);
     }
+}
+
+// flags: KF_FORCE / KF_SOLID when any domain of the batch has a volume force /
+// a solid node
+template <typename S, typename T, int UNI>
+inline cudaError_t launch_batch_flat_any(const Fused2Args<S, T> *doms, const FlatTile *tiles, int ntiles,
+                                         int parity, int flags, cudaStream_t s)
+{
+    constexpr int TY = FLAT_ROWS;
+    const dim3 grid(ntiles), block(32 * TY);
+    if (flags & KF_SOLID)
+        return launch_dependent(k_batch_flat<S, T, TY, KF_FORCE | KF_SOLID | UNI>, grid, block, 0, s, doms, tiles,
+                                parity);
+    if (flags & KF_FORCE)
+        return launch_dependent(k_batch_flat<S, T, TY, KF_FORCE>, grid, block, 0, s, doms, tiles, parity);
+    return launch_dependent(k_batch_flat<S, T, TY, 0>, grid, block, 0, s, doms, tiles, parity);
 }
 
 } // namespace sclbm

@@ -215,6 +215,9 @@ bool flat_fits(size_t nx, size_t ny);
 cudaError_t launch_flat2_fp64(const Fused2Args<double, double> &a, cudaStream_t s);
 cudaError_t launch_flat2_f32(const Fused2Args<float, float> &a, cudaStream_t s);
 cudaError_t launch_flat2_f16(const Fused2Args<__half, float> &a, cudaStream_t s);
+struct FlatTile;
+cudaError_t launch_batch_flat_fp64(const Fused2Args<double, double> *doms, const FlatTile *tiles, int ntiles,
+                                   int parity, int flags, cudaStream_t s);
 // `steps` <= K single-component steps in one launch (fused_single.cuh), K from
 // single_depth; lattices for which single_fits is false are refused
 bool single_fits(size_t nx, size_t ny);

@@ -8,5 +8,10 @@ cudaError_t launch_flat2_fp64(const Fused2Args<double, double> &a, cudaStream_t 
 {
     return launch_flat2_any<double, double, 0>(a, s);
 }
+cudaError_t launch_batch_flat_fp64(const Fused2Args<double, double> *doms, const FlatTile *tiles, int ntiles,
+                                   int parity, int flags, cudaStream_t s)
+{
+    return launch_batch_flat_any<double, double, 0>(doms, tiles, ntiles, parity, flags, s);
+}
 
 } // namespace sclbm
