@@ -485,8 +485,8 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
 // Whether the domain's steps run in pairs (fused_two.cuh): the shifted forms
 // beyond 450 k (FP32) or 1.5 M (FP16) nodes; below, where the buffers fit L2,
 // one node per thread is faster.  us per step, pairs / one node per thread:
-// FP32 600^2 11.3 / 10.0 (with solid nodes 12.4 / 12.3), 700^2 12.3 / 12.9 (14.4
-// / 15.8), 1024^2 22.6 / 31.6; FP16 1024^2 24.6 / 24.0 (27.8 / 26.3), 1200^2 33 /
+// FP32 600^2 11.3 / 10.0 (with solid nodes 12.4 / 12.3), 700^2 12.3 / 12.9 (14.3
+// / 15.7), 1024^2 21.5 / 31.6; FP16 1024^2 24.6 / 24.0 (27.8 / 26.3), 1200^2 33 /
 // 33 (39 / 37), 2048 x 1024 44 / 47.5 (52 / 52).  Lattices that need 64-bit
 // offsets, and domains with a variant or a tile width of the caller's choice,
 // take single steps; a band height of the caller's choice asks for pairs.

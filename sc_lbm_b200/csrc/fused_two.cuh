@@ -39,6 +39,7 @@
 // byte for byte.
 #pragma once
 #include "fused_step.cuh"
+#include "launch.cuh"
 
 namespace sclbm {
 
@@ -160,7 +161,13 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
 #pragma unroll
         for (int k = 0; k < 2; ++k)
 #pragma unroll
-            for (int i = 0; i < 9; ++i) f[k][i] = Store<S>::ld(a.fin[k] + elem<false>(i, a.N, node));
+            for (int i = 0; i < 9; ++i) {
+                // FP16 without solid nodes: the array's base first (280 -> 273 us
+                // on 4096^2: fewer wide multiplies on the FP32 pipe; no gain elsewhere)
+                const S *p = sizeof(S) == 2 && !SOLID ? a.fin[k] + (size_t)i * a.N + node
+                                                      : a.fin[k] + elem<false>(i, a.N, node);
+                f[k][i] = Load<S>::value(p);
+            }
     };
     // L2 is asked for the row after the one being loaded, one 128-byte line per
     // thread (FP16 289 -> 277 us a step, with solid nodes 343 -> 328; FP32 1-2 %; a
@@ -254,7 +261,8 @@ __device__ __forceinline__ void two_unit(const Fused2Args<S, float> &a, const in
 // (362 against 288 us on 4096^2).
 constexpr int TWO_CTAS = 4;
 
-// strip s covers the columns [s*w, min(nx, (s+1)*w)), band b the rows
+// Launched as a programmatic dependent (launch.cuh): 1024^2 22.6 -> 21.5 us a
+// step, 700^2 15.4 -> 14.3.  Strip s covers the columns [s*w, min(nx, (s+1)*w)), band b the rows
 // [b*ny/bands, (b+1)*ny/bands); neighbouring bands march in opposite
 // directions, so the rows they share are read by both near the same time
 template <typename S, int TX, int FLAGS>
@@ -265,6 +273,8 @@ __global__ void __launch_bounds__(TX, TWO_CTAS)
     const int band = blockIdx.y, xb = blockIdx.x * w;
     const int y0 = (int)((long long)band * a.ny / bands);
     const int nrow = (int)((long long)(band + 1) * a.ny / bands) - y0;
+    dependent_wait();
+    dependent_launch();
     two_unit<S, TX, FLAGS>(a, xb, min(w, a.nx - xb), y0, nrow, (band & 1) != 0, sh);
 }
 
@@ -326,8 +336,7 @@ inline cudaError_t launch_two2_f(const Fused2Args<S, float> &a, int rows, cudaSt
 {
     const int w = two_width(a.nx), strips = (a.nx + w - 1) / w;
     const int bands = std::min((a.ny + rows - 1) / rows, 65535);
-    k_two2<S, TX, FLAGS><<<dim3(strips, bands), TX, 0, s>>>(a, w, bands);
-    return cudaGetLastError();
+    return launch_dependent(k_two2<S, TX, FLAGS>, dim3(strips, bands), dim3(TX), 0, s, a, w, bands);
 }
 
 // rows: rows per band (0: two_rows); lattices with solid nodes run the uniform
@@ -355,7 +364,10 @@ struct TwoUnit {
 };
 
 // One CTA per unit, in the list's order (largest first): the block scheduler
-// balances them, no counter to take turns at.  doms holds two entries per
+// balances them, no counter to take turns at.  An ordinary launch: as a
+// programmatic dependent the next step's uneven units fill the free places
+// first, which put four on some SMs (eight mixed domains 9.2 -> 10.6 us a step,
+// others 1-3 % faster).  doms holds two entries per
 // domain (buffer parity 0 and 1); the unit's argument block is copied into
 // shared memory.
 template <typename S, int FLAGS>
