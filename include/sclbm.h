@@ -268,12 +268,16 @@ int sclbm_domain_step(sclbm_domain *d, int nsteps);
  * FP64 (out[3*comp + 0..2]); out[6] = number of non-finite populations. */
 int sclbm_domain_mass_momentum(sclbm_domain *d, double out[7]);
 /* Kernel selection (all variants give identical results):
- *   0 = automatic (default): the fastest measured form -- the ring kernel
- *       on lattices whose rows start on 16-byte boundaries and whose bands
- *       fill three waves of the GPU (FP64: the depth of 12 and 16-row bands;
- *       FP32: the depth of 13 and 24-row bands; FP16: the depth of 12 and
- *       32-row bands), else 8 for FP32/FP16 storage with solid nodes, 2
- *       otherwise;
+ *   0 = automatic (default): the fastest measured form -- one component:
+ *       several steps per launch; two components: two steps per launch for
+ *       FP32 beyond 450 k and FP16 beyond 1.5 M nodes, one node per thread
+ *       below and for FP64 up to 4 M nodes, the ring kernel (rows on 16-byte
+ *       boundaries; FP64: the depth of 12 and 16-row bands; FP32: the depth
+ *       of 13 and 24-row bands; FP16: the depth of 12 and 32-row bands) for
+ *       larger FP64 lattices and an odd last step.  With tile_y or threads of
+ *       the caller's choice: two steps per launch in bands of tile_y rows
+ *       (FP32, FP16), else the ring where its bands fill three waves of the
+ *       GPU, else 8 for FP32/FP16 storage with solid nodes, 2 otherwise;
  *   1 = two pass (density kernel, then the fused kernel reading it);
  *   2 = single pass, one tile per CTA, population rows held in registers;
  *   3 = single pass, population rows staged through a shared-memory ring by
@@ -458,8 +462,10 @@ typedef struct sclbm_batch sclbm_batch;
 int sclbm_batch_create(sclbm_domain *const *domains, int ndomains, const int *tile_y_per_domain,
                        sclbm_batch **out);
 void sclbm_batch_destroy(sclbm_batch *b);
-/* Work decomposition (same results either way): 0 = automatic (batches with
- * solid nodes: the body the autotuner's mixed-ensemble sweep found fastest
+/* Work decomposition (same results either way): 0 = automatic (FP32, FP16: two
+ * steps per launch, a CTA per strip and band; FP64 with solid nodes or fewer
+ * than 4 M nodes in all and no tile_y_per_domain: one node per thread; else,
+ * and for steps left over, batches with solid nodes: the body the autotuner's mixed-ensemble sweep found fastest
  * for the precision -- the ring body 11 with 16-row units for FP64, 24 for
  * FP32 and 32 for FP16; other batches: the tuned variant of the size
  * class holding most of the batch's nodes); 11 = ring body: persistent CTAs
