@@ -819,13 +819,13 @@ int sclbm_lbm_step_single(sclbm_lbm *l, const sclbm_geometry *g, sclbm_fluid *f,
     a.c.inv_omega = 1.0 / f->omega;
     a.c.force_on = force != nullptr;
     for (int i = 0; i < 9; ++i) a.c.force[i] = force ? force[i] : 0.0;
-    // several steps per launch; under capture odd ones, so that the arrays end
-    // where single steps would leave them
-    const bool several = single_fits(g->nx, g->ny), odd = several && being_captured(stream());
+    // several steps per launch; the fluid's and the LBM's arrays end as after
+    // single steps, for graphs that were captured from any of their operators
+    const bool several = single_fits(g->nx, g->ny);
     const int K = several ? single_depth(g->nx, g->ny, true) : 1;
-    for (int s = 0, n; s < nsteps; s += n) {
-        n = std::min(K, nsteps - s);
-        if (odd && n % 2 == 0) --n;
+    const int launches = single_launches(nsteps, K, true);
+    for (int s = 0, k = 0, n; k < launches; ++k, s += n) {
+        n = std::min(K, nsteps - s - (launches - 1 - k)); // a step at least for each to come
         a.fin = f->d[SCLBM_FIELD_F];
         a.fout = l->d_tmp[0];
         CUDA_LAUNCH(several ? launch_single_fp64(a, K, n, stream()) : launch_fused1_fp64(a, stream()));

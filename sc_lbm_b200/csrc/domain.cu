@@ -515,17 +515,21 @@ static int domain_launch_two(sclbm_domain *d, cudaStream_t s)
     return SCLBM_OK;
 }
 
+cudaStream_t domain_stream(sclbm_domain *d)
+{
+    cudaStream_t s = stream();
+    if (!d->held) d->held = being_captured(s);
+    return s;
+}
+
 // nsteps of a single-component domain, several per launch
 static int domain_single_steps(sclbm_domain *d, int nsteps, cudaStream_t s)
 {
     const int K = single_depth(d->nx, d->ny, d->prec == SCLBM_FP64);
-    // a graph has to find the state where it left it: odd launches turn the
-    // buffers over as often as their steps would
-    const bool odd = being_captured(s);
-    int rc = SCLBM_OK, done = 0, launches = 0;
-    while (done < nsteps) {
-        int n = std::min(K, nsteps - done);
-        if (odd && n % 2 == 0) --n;
+    const int launches = single_launches(nsteps, K, d->held);
+    int rc = SCLBM_OK, done = 0, k = 0;
+    for (; k < launches; ++k) {
+        const int n = std::min(K, nsteps - done - (launches - 1 - k)); // a step at least for each to come
         cudaError_t e;
         if (d->prec == SCLBM_FP64) {
             Fused1Args<double, double> a;
@@ -546,9 +550,8 @@ static int domain_single_steps(sclbm_domain *d, int nsteps, cudaStream_t s)
         }
         d->parity ^= 1;
         done += n;
-        ++launches;
     }
-    if ((done ^ launches) & 1) { // the parity counts steps
+    if ((done ^ k) & 1) { // the parity counts steps
         std::swap(d->buf[0], d->buf[1]);
         d->parity ^= 1;
     }
@@ -697,7 +700,7 @@ int sclbm_domain_step_rows(sclbm_domain *d, int row0, int nrows, int finish)
     if (row0 < 0 || nrows < 0 || (size_t)row0 + (size_t)nrows > d->ny)
         return set_error(SCLBM_E_OUT_OF_RANGE, "row range outside the domain");
     if (d->variant == 1) return set_error(SCLBM_E_INVALID_ARGUMENT, "row ranges need a single-pass variant");
-    cudaStream_t s = stream();
+    cudaStream_t s = domain_stream(d);
     if (nrows > 0) {
         // the register tile (in its uniform solid form for shifted lattices with solid nodes)
         const int v = d->has_solid && d->prec != SCLBM_FP64 ? 8 : 2;
@@ -970,15 +973,16 @@ int sclbm_domain_step(sclbm_domain *d, int nsteps)
     if (nsteps < 0) return set_error(SCLBM_E_INVALID_ARGUMENT, "negative step count");
     if (d->variant == 1 && d->ncomp == 2 && !d->rho_tmp[0])
         return set_error(SCLBM_E_RUNTIME, "two-pass buffers missing");
-    cudaStream_t s = stream();
+    cudaStream_t s = domain_stream(d);
     if (d->ncomp == 1 && single_fits(d->nx, d->ny)) return domain_single_steps(d, nsteps, s);
     int rc = SCLBM_OK, pairs = two_step(d) ? nsteps / 2 : 0;
     // The parity counts steps (a batch's domains have to be in step), and a pair
     // turns the buffers over once: after an odd number of pairs the two buffers
     // change names.  Where somebody holds their addresses -- a batch the domain
-    // is or was in, or a graph being captured, which has to find the state
-    // where it left it after an even number of steps -- the pairs are even.
-    if ((pairs & 1) && (d->batched || being_captured(s))) --pairs;
+    // is or was in, or a graph captured from a call on it, which has to find the
+    // state where it left it after an even number of steps, whenever it is
+    // replayed -- the pairs are even.
+    if ((pairs & 1) && d->held) --pairs;
     int done = 0;
     for (; done < pairs && !rc; ++done) rc = domain_launch_two(d, s);
     if (rc) --done; // the failed launch left the buffers as they were

@@ -21,13 +21,15 @@ struct sclbm_domain {
     int tile_y = 0;   // rows per tile (0: default)
     int tx = 128;     // threads per CTA
     bool has_solid = true; // the mask has solid nodes
-    bool batched = false;  // a batch holds, or once held, the buffers' addresses
+    bool held = false;     // a batch or a captured graph has the buffers' addresses, or once had them
     size_t bytes = 0; // device bytes held
 };
 
 namespace sclbm {
 size_t elem_size(sclbm_precision p);
 int domain_launch_step(sclbm_domain *d, cudaStream_t s);
+// the stream for work on d's buffers; notes on d when a graph is being captured there
+cudaStream_t domain_stream(sclbm_domain *d);
 int domain_refresh_codes(sclbm_domain *d, cudaStream_t s); // after the device mask has changed
 int domain_default_tile_y(const sclbm_domain *d);
 int domain_field_async(sclbm_domain *d, int comp, int what, double *host, cudaStream_t s);

@@ -173,7 +173,7 @@ extern "C" int sclbm_domain_write_text(sclbm_domain *d, int comp, int what, cons
     if (comp < 0 || comp >= d->ncomp) return set_error(SCLBM_E_INVALID_ARGUMENT, "bad component");
     if (what < 0 || what > 3) return set_error(SCLBM_E_INVALID_ARGUMENT, "what is 0..3");
     const size_t count = (what == 3 ? 9 : 1) * d->N;
-    cudaStream_t s = stream();
+    cudaStream_t s = domain_stream(d);
     PinnedJob job;
     cudaError_t e = cudaMallocHost(&job.host, count * sizeof(double));
     if (e != cudaSuccess) {

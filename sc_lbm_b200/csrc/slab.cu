@@ -56,7 +56,7 @@ int halo_copy(sclbm_domain *d, int rows, int side, void *buf, bool unpack)
     const int threads = 256;
     const int blocks = (int)std::min<size_t>((total + threads - 1) / threads, 148 * 16);
     void *f0 = d->buf[d->parity][0], *f1 = d->ncomp > 1 ? d->buf[d->parity][1] : f0;
-    cudaStream_t s = stream();
+    cudaStream_t s = domain_stream(d);
     switch (elem_size(d->prec)) {
     case 8:
         k_halo<uint64_t><<<blocks, threads, 0, s>>>((uint64_t *)f0, (uint64_t *)f1, (uint64_t *)buf,
@@ -175,7 +175,7 @@ int halo_min_copy(sclbm_domain *d, int side, void *buf, bool unpack)
     const int threads = 256;
     const int blocks = (int)std::min<size_t>((total + threads - 1) / threads, 148 * 16);
     void *f0 = d->buf[d->parity][0], *f1 = d->ncomp > 1 ? d->buf[d->parity][1] : f0;
-    cudaStream_t s = stream();
+    cudaStream_t s = domain_stream(d);
     switch (elem_size(d->prec)) {
     case 8:
         k_halo_min<uint64_t><<<blocks, threads, 0, s>>>((uint64_t *)f0, (uint64_t *)f1, (uint64_t *)buf,
