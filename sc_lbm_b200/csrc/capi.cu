@@ -359,7 +359,6 @@ int sclbm_fluid_create(size_t nx, size_t ny, double tau, sclbm_fluid **out)
     if (rc) return rc;
     auto *f = new (std::nothrow) sclbm_fluid();
     if (!f) return set_error(SCLBM_E_ALLOC, "host allocation failed");
-    host_copy_retain();
     f->nx = nx;
     f->ny = ny;
     f->N = nx * ny;
@@ -384,7 +383,6 @@ void sclbm_fluid_destroy(sclbm_fluid *f)
     for (auto *p : f->d)
         if (p) cudaFree(p);
     delete f;
-    host_copy_release();
 }
 
 int sclbm_fluid_set_interactions(sclbm_fluid *f, double g_solid, double g_fluid)

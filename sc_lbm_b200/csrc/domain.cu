@@ -610,7 +610,6 @@ void sclbm_domain_destroy(sclbm_domain *d)
     if (d->partials) cudaFree(d->partials);
     if (d->d_status) cudaFree(d->d_status);
     delete d;
-    host_copy_release();
 }
 
 int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_params *p,
@@ -637,7 +636,6 @@ int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_p
     }
     auto *d = new (std::nothrow) sclbm_domain();
     if (!d) return set_error(SCLBM_E_ALLOC, "host allocation failed");
-    host_copy_retain();
     d->nx = nx;
     d->ny = ny;
     d->N = N;
@@ -843,7 +841,7 @@ int sclbm_domain_download_f(sclbm_domain *d, int comp, double *f, size_t count)
         SCLBM_CUDA(copy_to_host(f, src, 9 * d->N * 8, s));
     } else {
         const double rr = d->p.rho_ref[comp];
-        const bool bounced = host_copy_bounced(f, d->N * 8);
+        host_pages_in(f, 9 * d->N * 8);
         for (int i = 0; i < 9; ++i) {
             if (d->prec == SCLBM_FP32_SHIFTED)
                 k_download_dir<float><<<grid_for(d->N, 256), 256, 0, s>>>(
@@ -852,9 +850,7 @@ int sclbm_domain_download_f(sclbm_domain *d, int comp, double *f, size_t count)
                 k_download_dir<__half><<<grid_for(d->N, 256), 256, 0, s>>>(
                     d->N, d->d_mask, (const __half *)src + i * d->N, d->staging, w_eq(i) * rr);
             SCLBM_LAUNCHED("download conversion");
-            if (bounced) SCLBM_CUDA(copy_to_host(f + i * d->N, d->staging, d->N * 8, s));
-            else
-                SCLBM_CUDA(cudaMemcpyAsync(f + i * d->N, d->staging, d->N * 8, cudaMemcpyDeviceToHost, s));
+            SCLBM_CUDA(cudaMemcpyAsync(f + i * d->N, d->staging, d->N * 8, cudaMemcpyDeviceToHost, s));
         }
         SCLBM_CUDA(cudaStreamSynchronize(s));
     }
@@ -956,11 +952,8 @@ int sclbm_domain_download_velocity(sclbm_domain *d, int comp, double *ux, double
     default: k_velocity<__half><<<g, 256, 0, s>>>(d->N, d->d_mask, (const __half *)src, a, b, rr, 1); break;
     }
     SCLBM_LAUNCHED("velocity");
-    if (host_copy_bounced(ux, d->N * 8)) {
-        SCLBM_CUDA(copy_to_host(ux, a, d->N * 8, s));
-        SCLBM_CUDA(copy_to_host(uy, b, d->N * 8, s));
-        return SCLBM_OK;
-    }
+    host_pages_in(ux, d->N * 8);
+    host_pages_in(uy, d->N * 8);
     SCLBM_CUDA(cudaMemcpyAsync(ux, a, d->N * 8, cudaMemcpyDeviceToHost, s));
     SCLBM_CUDA(cudaMemcpyAsync(uy, b, d->N * 8, cudaMemcpyDeviceToHost, s));
     SCLBM_CUDA(cudaStreamSynchronize(s));

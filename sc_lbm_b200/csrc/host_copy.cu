@@ -1,183 +1,86 @@
 // host_copy.cu -- device to host copies of whole fields.
 //
-// A copy into pageable memory goes through the driver's own staging and one
-// host thread, which on freshly allocated arrays spends most of the time on
-// page faults (2.7 GB/s on 9.4 MB).  Here the chunks of a large copy land in a
-// small pinned buffer while a few threads move the chunks before them into the
-// caller's array.  Measured with 16 cores, driver / here: two fresh arrays of
-// 4.7 MB 3.3 / 1.1-1.4 ms, of 75 MB 32 / 11 ms; an array in use 4.7 MB 0.26 / 0.23
-// ms, 75 MB 3.6 / 2.7 ms (four threads: 75 MB fresh 16 ms).
+// A freshly allocated array has no pages behind it: copied into as it is, the
+// driver's one copying thread takes a page fault every 4 KB, after the stream
+// has done its work (2.0 GB/s, against 19 into an array in use).  Here its pages
+// are asked for first, while the stream still works, by up to four threads for
+// larger arrays; the copy itself is the driver's.  Nothing is kept between
+// calls: a pinned buffer that a copy passes through costs 20 ms to allocate,
+// which a program that reads one field of an object never gets back.
 //
-// The pinned buffer (16 MB) belongs to the process while any domain or fluid is
-// alive: it is allocated by the first copy that needs it and freed with the
-// last object.  One copy uses it at a time; another thread's copy meanwhile
-// takes the driver's path.
+// Measured with 16 cores, ms without / with (alone; behind steps that take
+// longer than the pages): 4.7 MB 2.3 / 1.5; 2.3 / 0.29, 9.7 MB 4.8 / 2.5; 4.7 /
+// 0.84, 75 MB 36.9 / 11.8.  An array in use, 4.7 MB: 0.27 / 0.27.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
-#include <atomic>
-#include <cstring>
-#include <mutex>
+#include <cstdint>
 #include <system_error>
 #include <thread>
 
 #include "internal.h"
 
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23 // Linux 5.14
+#endif
+
 namespace sclbm {
 
 namespace {
-constexpr size_t CHUNK = size_t(512) << 10;
-constexpr int SLOTS = 32;
-constexpr int THREADS = 8; // at most, and half the cores
-// smaller copies: the driver's path (1.6 MB: 0.14 ms, and 0.4 with threads to start)
-constexpr size_t LEAST = size_t(3) << 20;
+constexpr size_t LEAST = size_t(3) << 20;  // smaller arrays: malloc hands out pages in use
+constexpr size_t SHARE = size_t(4) << 20;  // per thread; starting one takes as long as 0.3 MB of pages
+constexpr int THREADS = 4;                 // eight were slower (75 MB 15.9 ms)
 
-std::mutex g_mu; // the buffer and its events
-char *g_buf = nullptr;
-cudaEvent_t g_ev[SLOTS] = {};
-int g_dev = -1;
-std::atomic<long> g_objects{0};
-
-void release_locked()
+// whether some of the page-aligned range has no pages yet, by five of them
+bool pages_missing(char *a, size_t len, size_t page)
 {
-    for (auto &e : g_ev)
-        if (e) {
-            cudaEventDestroy(e);
-            e = nullptr;
-        }
-    if (g_buf) cudaFreeHost(g_buf);
-    g_buf = nullptr;
-    g_dev = -1;
-}
-
-// the buffer and events of the current device; false: not to be had
-bool acquire_locked(int dev)
-{
-    if (g_buf && g_dev == dev) return true;
-    release_locked();
-    bool ok = cudaHostAlloc((void **)&g_buf, CHUNK * SLOTS, cudaHostAllocPortable) == cudaSuccess;
-    for (auto &e : g_ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-    g_dev = dev;
-    if (!ok) {
-        cudaGetLastError();
-        release_locked();
+    for (int k = 0; k < 5; ++k) {
+        unsigned char in = 1;
+        const size_t at = (len / page - 1) * k / 4 * page;
+        if (mincore(a + at, page, &in) == 0 && !(in & 1)) return true;
     }
-    return ok;
-}
-
-cudaError_t plain_copy(void *dst, const void *src, size_t bytes, cudaStream_t s)
-{
-    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
-    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
-}
-
-// One copy through the buffer: chunk i passes through slot i % SLOTS, its
-// arrival marked by the slot's event; whoever has emptied a slot requests the
-// chunk that comes next there.
-struct Transfer {
-    char *dst;
-    const char *src;
-    size_t bytes;
-    cudaStream_t s;
-    int dev, chunks;
-    std::atomic<int> next{0}, requested{0}, error{cudaSuccess};
-
-    size_t size(int i) const { return std::min(CHUNK, bytes - (size_t)i * CHUNK); }
-    void fail(cudaError_t e)
-    {
-        int none = cudaSuccess;
-        error.compare_exchange_strong(none, e);
-    }
-    void request(int i)
-    {
-        cudaError_t e = cudaMemcpyAsync(g_buf + (size_t)(i % SLOTS) * CHUNK, src + (size_t)i * CHUNK, size(i),
-                                        cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaEventRecord(g_ev[i % SLOTS], s);
-        if (e != cudaSuccess) fail(e);
-    }
-    void work()
-    {
-        for (int i; (i = next.fetch_add(1)) < chunks;) {
-            // chunks are requested in order: a slot is emptied before the
-            // request of the chunk after it, by a thread that waits for no one
-            while (requested.load() <= i) {
-                if (error.load() != cudaSuccess) return;
-                std::this_thread::yield();
-            }
-            if (error.load() != cudaSuccess) return;
-            const cudaError_t e = cudaEventSynchronize(g_ev[i % SLOTS]);
-            if (e != cudaSuccess) return fail(e);
-            std::memcpy(dst + (size_t)i * CHUNK, g_buf + (size_t)(i % SLOTS) * CHUNK, size(i));
-            if (i + SLOTS < chunks) {
-                while (requested.load() < i + SLOTS) { // in order
-                    if (error.load() != cudaSuccess) return;
-                    std::this_thread::yield();
-                }
-                request(i + SLOTS);
-                requested.store(i + SLOTS + 1);
-            }
-        }
-    }
-};
-
-cudaError_t bounced_copy(Transfer &t)
-{
-    const int first = std::min(t.chunks, SLOTS);
-    for (int i = 0; i < first; ++i) t.request(i);
-    t.requested.store(first);
-    // whatever the stream had to do before the copy is waited for here, by one thread
-    if (t.error.load() == cudaSuccess) {
-        const cudaError_t e = cudaEventSynchronize(g_ev[0]);
-        if (e != cudaSuccess) t.fail(e);
-    }
-    std::thread helpers[THREADS - 1];
-    const int cores = (int)std::thread::hardware_concurrency();
-    const int want = std::min({THREADS - 1, t.chunks - 1, std::max(0, cores / 2 - 1)});
-    int n = 0;
-    try {
-        for (; n < want; ++n)
-            helpers[n] = std::thread([&t] {
-                const cudaError_t e = cudaSetDevice(t.dev);
-                if (e != cudaSuccess) return t.fail(e);
-                t.work();
-            });
-    } catch (const std::system_error &) {
-        // fewer helpers: the others claim their chunks
-    }
-    t.work();
-    for (int k = 0; k < n; ++k) helpers[k].join();
-    const cudaError_t e = cudaStreamSynchronize(t.s); // after an error: no copy may still be under way
-    return t.error.load() != cudaSuccess ? (cudaError_t)t.error.load() : e;
+    return false;
 }
 } // namespace
 
-void host_copy_retain() { g_objects.fetch_add(1); }
-void host_copy_release()
-{
-    if (g_objects.fetch_sub(1) != 1) return;
-    std::lock_guard<std::mutex> lk(g_mu);
-    if (g_objects.load() == 0) release_locked();
-}
-
-bool host_copy_bounced(const void *dst, size_t bytes)
+void host_pages_in(void *dst, size_t bytes)
 {
     cudaPointerAttributes at{};
-    if (bytes < LEAST) return false;
-    if (cudaPointerGetAttributes(&at, dst) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
-    cudaGetLastError();
-    return false;
+    if (bytes < LEAST) return;
+    if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t first = ((uintptr_t)dst + page - 1) / page * page, end = ((uintptr_t)dst + bytes) / page * page;
+    if (end <= first) return;
+    char *const a = (char *)first;
+    const size_t len = end - first;
+    if (!pages_missing(a, len, page)) return;
+    const int cores = (int)std::thread::hardware_concurrency();
+    const int n = std::max(1, std::min({THREADS, cores / 2, (int)std::min<size_t>(len / SHARE, THREADS)}));
+    // a failure (an older kernel, an odd mapping) leaves the faults to the copy
+    auto part = [=](int k) {
+        const size_t b = len / page * k / n * page, e = len / page * (k + 1) / n * page;
+        madvise(a + b, e - b, MADV_POPULATE_WRITE);
+    };
+    std::thread helpers[THREADS];
+    int k = 1;
+    try {
+        for (; k < n; ++k) helpers[k] = std::thread(part, k);
+    } catch (const std::system_error &) { // no more threads: the copy takes these faults
+    }
+    part(0);
+    for (int j = 1; j < k; ++j) helpers[j].join();
 }
 
 cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t s)
 {
-    if (!host_copy_bounced(dst, bytes)) return plain_copy(dst, src, bytes, s);
-    int dev = 0;
-    if (being_captured(s) || cudaGetDevice(&dev) != cudaSuccess) return plain_copy(dst, src, bytes, s);
-    std::unique_lock<std::mutex> lk(g_mu, std::try_to_lock);
-    if (!lk.owns_lock() || !acquire_locked(dev)) {
-        if (lk.owns_lock()) lk.unlock();
-        return plain_copy(dst, src, bytes, s);
-    }
-    Transfer t{(char *)dst, (const char *)src, bytes, s, dev, (int)((bytes + CHUNK - 1) / CHUNK)};
-    return bounced_copy(t);
+    host_pages_in(dst, bytes);
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
 }
 
 } // namespace sclbm

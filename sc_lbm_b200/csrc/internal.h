@@ -32,12 +32,10 @@ cudaStream_t stream();
 int ensure_device();
 int grid_for(size_t n, int block);  // grid-stride grid size (multiple of the SM count)
 int sm_count();
-// device to host, complete on return (host_copy.cu); retain/release: every
-// object whose fields may be copied out, while it lives
+// device to host, complete on return, and the pages of a destination asked for
+// while the stream works (host_copy.cu)
 cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t s);
-bool host_copy_bounced(const void *dst, size_t bytes); // pageable and large: else a queued copy is as good
-void host_copy_retain();
-void host_copy_release();
+void host_pages_in(void *dst, size_t bytes);
 bool being_captured(cudaStream_t s); // work queued on s goes into a graph, or cannot be told not to
 
 // ------------------------------------------------------------- host geometry
