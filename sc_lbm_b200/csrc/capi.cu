@@ -10,6 +10,7 @@
 #include "domain.h"
 #include "internal.h"
 #include "ops_fp64.h"
+#include "routes.h"
 
 namespace sclbm {
 
@@ -820,13 +821,14 @@ int sclbm_lbm_step_single(sclbm_lbm *l, const sclbm_geometry *g, sclbm_fluid *f,
     // several steps per launch; the fluid's and the LBM's arrays end as after
     // single steps, for graphs that were captured from any of their operators
     const bool several = single_fits(g->nx, g->ny);
-    const int K = several ? single_depth(g->nx, g->ny, true) : 1;
+    const int K = several ? single_depth(g->nx, g->ny, SCLBM_FP64, sm_count()) : 1;
+    const bool one = single_pays(g->nx, g->ny, SCLBM_FP64, K, 1);
     const int launches = single_launches(nsteps, K, true);
     for (int s = 0, k = 0, n; k < launches; ++k, s += n) {
         n = std::min(K, nsteps - s - (launches - 1 - k)); // a step at least for each to come
         a.fin = f->d[SCLBM_FIELD_F];
         a.fout = l->d_tmp[0];
-        CUDA_LAUNCH(several ? launch_single_fp64(a, K, n, stream()) : launch_fused1_fp64(a, stream()));
+        CUDA_LAUNCH(n > 1 || one ? launch_single_fp64(a, K, n, stream()) : launch_fused1_fp64(a, stream()));
         std::swap(f->d[SCLBM_FIELD_F], l->d_tmp[0]);
     }
     return SCLBM_OK;

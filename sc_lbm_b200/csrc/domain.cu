@@ -16,6 +16,7 @@
 
 #include "domain.h"
 #include "fused_step.cuh"
+#include "routes.h"
 
 namespace sclbm {
 
@@ -525,7 +526,8 @@ cudaStream_t domain_stream(sclbm_domain *d)
 // nsteps of a single-component domain, several per launch
 static int domain_single_steps(sclbm_domain *d, int nsteps, cudaStream_t s)
 {
-    const int K = single_depth(d->nx, d->ny, d->prec == SCLBM_FP64);
+    const int K = single_depth(d->nx, d->ny, d->prec, sm_count());
+    const bool one = single_pays(d->nx, d->ny, d->prec, K, 1);
     const int launches = single_launches(nsteps, K, d->held);
     int rc = SCLBM_OK, done = 0, k = 0;
     for (; k < launches; ++k) {
@@ -534,15 +536,15 @@ static int domain_single_steps(sclbm_domain *d, int nsteps, cudaStream_t s)
         if (d->prec == SCLBM_FP64) {
             Fused1Args<double, double> a;
             fill1(d, a);
-            e = launch_single_fp64(a, K, n, s);
+            e = n > 1 || one ? launch_single_fp64(a, K, n, s) : launch_fused1_fp64(a, s);
         } else if (d->prec == SCLBM_FP32_SHIFTED) {
             Fused1Args<float, float> a;
             fill1(d, a);
-            e = launch_single_f32(a, K, n, s);
+            e = n > 1 || one ? launch_single_f32(a, K, n, s) : launch_fused1_f32(a, s);
         } else {
             Fused1Args<__half, float> a;
             fill1(d, a);
-            e = launch_single_f16(a, K, n, s);
+            e = n > 1 || one ? launch_single_f16(a, K, n, s) : launch_fused1_f16(a, s);
         }
         if (e != cudaSuccess) {
             rc = cuda_fail(e, "single-component step launch");

@@ -217,17 +217,9 @@ struct FlatTile;
 cudaError_t launch_batch_flat_fp64(const Fused2Args<double, double> *doms, const FlatTile *tiles, int ntiles,
                                    int parity, int flags, cudaStream_t s);
 // `steps` <= K single-component steps in one launch (fused_single.cuh), K from
-// single_depth; lattices for which single_fits is false are refused
+// single_depth (routes.h) and not 1; lattices for which single_fits is false are
+// refused
 bool single_fits(size_t nx, size_t ny);
-int single_depth(size_t nx, size_t ny, bool fp64);
-// launches for nsteps, at most K each; keep: an odd number of them exactly when
-// nsteps is odd, so that two buffers in turn end as after single steps (one
-// more launch at most)
-inline int single_launches(int nsteps, int K, bool keep)
-{
-    const int n = nsteps / K + (nsteps % K != 0);
-    return keep && ((n ^ nsteps) & 1) ? n + 1 : n;
-}
 cudaError_t launch_single_fp64(const Fused1Args<double, double> &a, int K, int steps, cudaStream_t s);
 cudaError_t launch_single_f32(const Fused1Args<float, float> &a, int K, int steps, cudaStream_t s);
 cudaError_t launch_single_f16(const Fused1Args<__half, float> &a, int K, int steps, cudaStream_t s);

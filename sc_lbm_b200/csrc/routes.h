@@ -1,0 +1,74 @@
+// routes.h -- which kernel a call's steps run, by sizes and precision alone
+// (host rules without CUDA calls).
+#pragma once
+#include <algorithm>
+#include <cstddef>
+
+#include "sclbm.h"
+
+namespace sclbm {
+
+// ------------------------------------------------- single-component lattices
+// A launch of k_single (fused_single.cuh) takes as long as its tiles of 32 x 16
+// nodes with halo, however few nodes of their own they hold: 0.7 us and, per
+// tile, a + b n ns for n steps.  A tile of fewer rows costs less (8 + rows of
+// 24), one of fewer columns does not.  A step of the kernel with one node per
+// thread takes 4.2 us and c ns per node.  Measured us per step by tiles / by
+// nodes: FP64 2048^2 78 / 116, 29 x 40000 23 / 35, 33 x 30000 32 / 31, 4 x 100000
+// 49 / 10.4; FP32 2048^2 49 / 73, 29 x 40000 25.5 / 20.6, 4 x 100000 31 / 9.7; FP16
+// 2048^2 55 / 76, 33 x 30000 21.8 / 18.6; one step a call: FP64 500^2 9.0 / 9.4,
+// 1024^2 37.4 / 34.6, FP32 500^2 6.7 / 8.4, 1024^2 20.9 / 19.0.
+struct SingleCost {
+    int K;          // steps per launch on lattices of many tiles
+    double a, b, c; // ns
+};
+inline SingleCost single_cost(sclbm_precision p)
+{
+    if (p == SCLBM_FP64) return {2, 10.6, 2.4, 0.025};
+    if (p == SCLBM_FP32_SHIFTED) return {3, 5.0, 2.15, 0.0135};
+    return {3, 5.3, 2.5, 0.0155};
+}
+
+// whether n steps of the lattice in one launch of depth K beat n launches of
+// one node per thread; lattices whose tiles of a greater depth than K fit the
+// GPU at once: always (3.5 us against 4.2 for a single step)
+inline bool single_pays(size_t nx, size_t ny, sclbm_precision p, int K, int n)
+{
+    const SingleCost s = single_cost(p);
+    if (K > s.K) return true;
+    if (K < s.K) return false;
+    const size_t H = K - 1, w = 32 - 2 * H, h = 16 - 2 * H, rest = ny % h;
+    const double tiles = (double)((nx + w - 1) / w) * ((double)(ny / h) + (rest ? (8 + rest + 2 * H) / 24.0 : 0.0));
+    return 700 + tiles * (s.a + s.b * n) < n * (4200 + s.c * (double)nx * (double)ny);
+}
+
+// Steps per launch.  While the tiles of six steps (22 x 6 nodes) fit the GPU at
+// once (wave: two CTAs per SM) a launch's latency is worth the halo's work;
+// then five steps for the shifted forms up to one and a half waves of their
+// tiles (24 x 8), three for FP64 up to one wave (28 x 12), and as many as pay for
+// the repeated halo: three for the shifted forms, two for FP64, or one (no
+// tiles at all) on lattices a few nodes wide.  us per step for K = 2 / 3 / 5 / 6:
+// FP64 200 x 50 2.16 / 1.74 / 1.36 / 1.23, 400 x 200 3.07 / 2.66 / 2.81 / 3.85, 1500 x
+// 600 18.5 / 19.0 / 24.7 / 32.6; FP32 200 x 50 1.64 / 1.31 / 0.96 / 0.85, 400 x 200
+// 2.29 / 2.33 / 1.77 / 2.38, 1500 x 600 12.9 / 11.2 / 14.5 / 18.9.
+inline int single_depth(size_t nx, size_t ny, sclbm_precision p, int sms)
+{
+    const size_t wave = 2 * (size_t)sms;
+    auto tiles = [&](size_t w, size_t h) { return ((nx + w - 1) / w) * ((ny + h - 1) / h); };
+    if (tiles(22, 6) <= wave) return 6;
+    if (p == SCLBM_FP64 && tiles(28, 12) <= wave) return 3;
+    if (p != SCLBM_FP64 && tiles(24, 8) <= wave + wave / 2) return 5;
+    const int K = single_cost(p).K;
+    return single_pays(nx, ny, p, K, K) ? K : 1;
+}
+
+// launches for nsteps, at most K each; keep: an odd number of them exactly when
+// nsteps is odd, so that two buffers in turn end as after single steps (one
+// more launch at most)
+inline int single_launches(int nsteps, int K, bool keep)
+{
+    const int n = nsteps / K + (nsteps % K != 0);
+    return keep && ((n ^ nsteps) & 1) ? n + 1 : n;
+}
+
+} // namespace sclbm

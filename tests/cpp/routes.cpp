@@ -1,0 +1,28 @@
+// Answers of the library's dispatch rules (sc_lbm_b200/csrc/routes.h), one line
+// per question on standard input.
+#include <iostream>
+#include <string>
+
+#include "routes.h"
+
+using namespace sclbm;
+
+int main()
+{
+    std::string what;
+    while (std::cin >> what) {
+        size_t nx, ny;
+        int p, sms, n, K, keep;
+        if (what == "single") { // depth, and whether one step goes by tiles
+            std::cin >> nx >> ny >> p >> sms;
+            K = single_depth(nx, ny, (sclbm_precision)p, sms);
+            std::cout << K << ' ' << single_pays(nx, ny, (sclbm_precision)p, K, 1) << '\n';
+        } else if (what == "launches") {
+            std::cin >> n >> K >> keep;
+            std::cout << single_launches(n, K, keep != 0) << '\n';
+        } else {
+            return 1;
+        }
+    }
+    return 0;
+}

@@ -1,0 +1,62 @@
+"""Dispatch rules (sc_lbm_b200/csrc/routes.h), compiled from the library's own
+header: the kernel chosen is the faster one where both were timed on a B200."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+FP64, FP32, FP16, SMS = 0, 1, 2, 148
+
+
+@pytest.fixture(scope="module")
+def ask(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("routes") / "routes")
+    subprocess.run(["g++", "-std=c++17", "-I" + os.path.join(ROOT, "include"),
+                    "-I" + os.path.join(ROOT, "sc_lbm_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "cpp", "routes.cpp"), "-o", exe], check=True)
+
+    def answers(questions):
+        text = "\n".join(" ".join(map(str, q)) for q in questions)
+        out = subprocess.run([exe], input=text, check=True, capture_output=True, text=True).stdout
+        got = [tuple(map(int, line.split())) for line in out.splitlines()]
+        assert len(got) == len(questions)
+        return got
+    return answers
+
+
+# nx, ny, form: us per step of the depth, and by one node per thread (many
+# steps a call; one step a call)
+SINGLE = [
+    ((200, 50, FP64), 6, True), ((64, 32, FP32), 6, True), ((300, 300, FP64), 3, True),
+    ((400, 200, FP32), 5, True), ((400, 200, FP16), 5, True),
+    ((1500, 600, FP64), 2, False),     # 18.5 / 28.9; 32.0 / 28.9
+    ((2048, 2048, FP64), 2, False),    # 78 / 116; 135 / 116
+    ((1024, 1024, FP32), 3, False),    # 12.7 / 18.7; 20.9 / 19.0
+    ((2048, 2048, FP16), 3, False),    # 55 / 76; 99 / 76
+    ((500, 500, FP64), 2, True),       # 6.0 / 9.3; 9.0 / 9.4
+    ((500, 500, FP32), 3, True),       # 3.9 / 8.3; 6.7 / 8.4
+    ((29, 40000, FP64), 2, False),     # 23 / 35; 39 / 35
+    ((100000, 13, FP32), 3, False),    # 21.0 / 23.7; 38 / 24
+    ((4, 100000, FP64), 1, False),     # 49 / 10.4
+    ((4, 100000, FP32), 1, False),     # 31 / 9.7
+    ((4, 100000, FP16), 1, False),     # 36 / 10.4
+    ((29, 40000, FP32), 1, False),     # 25.5 / 20.6
+    ((33, 30000, FP16), 1, False),     # 21.8 / 18.6
+    ((200000, 4, FP64), 1, False),     # 32 / 25
+    ((1, 10000, FP64), 1, False),      # 6.7 / 4.3
+]
+
+
+def test_single_component_depth(ask):
+    got = ask([("single", *shape, SMS) for shape, _, _ in SINGLE])
+    assert got == [(depth, int(one)) for _, depth, one in SINGLE]
+
+
+def test_launch_counts(ask):
+    """Enough launches, none without a step, and on demand of the steps' parity."""
+    questions = [(n, K, keep) for n in range(0, 40) for K in (1, 2, 3, 5, 6) for keep in (0, 1)]
+    for (n, K, keep), (launches,) in zip(questions, ask([("launches", *q) for q in questions])):
+        least = -(-n // K)
+        assert least <= launches <= min(n, least + keep)
+        assert not keep or (launches - n) % 2 == 0
