@@ -428,9 +428,10 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
         if (e != cudaSuccess) return e;
     }
     // variant 0 picks the fastest measured form on B200: one node per thread,
-    // or the ring kernel (rows streamed into shared memory by tensor copies)
-    // at the depth and band height of ring_choice on large lattices whose rows
-    // start on 16-byte boundaries.  A tile height or width of the caller's
+    // the ring kernel (rows streamed into shared memory by tensor copies) at the
+    // depth and band height of ring_choice on large lattices whose rows start on
+    // 16-byte boundaries, or the register tile on large ones whose rows do not
+    // (routes.h).  A tile height or width of the caller's
     // choice asks for marching tiles: the ring where it fits and fills the
     // GPU, else the register tile, in its uniform solid form where FP32/FP16
     // lattices have solid nodes.  3 and 9 force the pipelined kernel; 11, 12,
@@ -438,7 +439,7 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
     // lattices: the register tile)
     const bool ring = d->variant == 0 && ring_row_aligned(d) && ring_fills_device(d);
     if (d->variant == 0 && d->tile_y == 0 && d->tx == 128 && flat_fits(d->nx, d->ny) &&
-        (!ring || flat_beats_ring(d))) {
+        (ring ? flat_beats_ring(d) : flat_beats_tile(d->nx, d->ny, d->prec, d->has_solid))) {
         if constexpr (sizeof(S) == 8) return launch_flat2_fp64(a, s);
         else if constexpr (sizeof(S) == 4) return launch_flat2_f32(a, s);
         else return launch_flat2_f16(a, s);

@@ -8,6 +8,26 @@
 
 namespace sclbm {
 
+// --------------------------------------------------- two-component lattices
+// Single steps on lattices that the ring kernel does not take: one node per
+// thread, or the register tile.  The tile keeps its rate on large lattices
+// where the halo loads of one node per thread come from DRAM; it loses the
+// columns that its last strip of 126 does not have.  us per step, one node per
+// thread / register tile: FP32 1200 x 1100 40.4 / 44.7, 1800 x 1500 78.8 / 84.9, 1500 x
+// 1100 52.4 / 50.1 (99 % of its strips full), 2047^2 123 / 118, 4095^2 484 / 450,
+// with disks 2801 x 2401 226 / 233, 3501 x 3001 355 / 351; FP16 2801 x 2401 145 / 155,
+// 3001 x 2701 184 / 176, with disks 4095^2 431 / 463; FP64 1501 x 1101 84 / 96, 4095^2
+// 808 / 953.
+inline bool flat_beats_tile(size_t nx, size_t ny, sclbm_precision p, bool solid)
+{
+    const size_t n = nx * ny, M = 1000000;
+    if (p == SCLBM_FP64) return true;
+    if (p == SCLBM_FP16_SHIFTED) return solid || n < 7 * M;
+    if (solid) return n < 9 * M;
+    const double full = (double)nx / (double)((nx + 125) / 126 * 126);
+    return n < 3 * M / 2 || (n < 3 * M && full < 0.985);
+}
+
 // ------------------------------------------------- single-component lattices
 // A launch of k_single (fused_single.cuh) takes as long as its tiles of 32 x 16
 // nodes with halo, however few nodes of their own they hold: 0.7 us and, per

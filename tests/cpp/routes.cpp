@@ -20,6 +20,9 @@ int main()
         } else if (what == "launches") {
             std::cin >> n >> K >> keep;
             std::cout << single_launches(n, K, keep != 0) << '\n';
+        } else if (what == "flat") { // one node per thread rather than the register tile
+            std::cin >> nx >> ny >> p >> keep;
+            std::cout << flat_beats_tile(nx, ny, (sclbm_precision)p, keep != 0) << '\n';
         } else {
             return 1;
         }

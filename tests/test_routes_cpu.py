@@ -60,3 +60,22 @@ def test_launch_counts(ask):
         least = -(-n // K)
         assert least <= launches <= min(n, least + keep)
         assert not keep or (launches - n) % 2 == 0
+
+
+# nx, ny, form, solid nodes: whether one node per thread was faster than the
+# register tile (us per step)
+FLAT = [
+    ((1021, 763, FP32, 0), True), ((1201, 1101, FP32, 0), True),    # 40.7 / 44.8
+    ((1801, 1501, FP32, 0), True),                                  # 82.4 / 84.7
+    ((1501, 1101, FP32, 0), False), ((1500, 1100, FP32, 0), False), # 53.2 / 50.2; 52.4 / 50.1
+    ((2047, 2047, FP32, 0), False), ((4095, 4095, FP32, 0), False), # 123 / 118; 484 / 450
+    ((2047, 2047, FP32, 1), True), ((2801, 2401, FP32, 1), True),   # 142 / 150; 226 / 233
+    ((3501, 3001, FP32, 1), False), ((4095, 4095, FP32, 1), False), # 355 / 351; 546 / 534
+    ((2801, 2401, FP16, 0), True), ((3001, 2701, FP16, 0), False),  # 145 / 155; 184 / 176
+    ((4095, 4095, FP16, 1), True),                                  # 431 / 463
+    ((1501, 1101, FP64, 0), True), ((4095, 4095, FP64, 1), True),   # 84 / 96; 967 / 1077
+]
+
+
+def test_single_steps_off_the_ring(ask):
+    assert ask([("flat", *q) for q, _ in FLAT]) == [(int(want),) for _, want in FLAT]
