@@ -22,6 +22,7 @@
 #include "fused_flat.cuh"
 #include "fused_ring.cuh"
 #include "fused_two.cuh"
+#include "routes.h"
 #include "tuning.h"
 
 
@@ -221,13 +222,14 @@ static int upload_args(sclbm_batch *b, const std::vector<int> &ty, const std::ve
 
 // Units of the two-step kernel: per domain its strips and bands, all of about
 // the rows that two_cost finds best for the batch's units (the caller's height
-// where given).  64 mixed domains, before the node codes: 24 rows 80 us per
+// where given; none when one of those is too low for pairs).  64 mixed domains, before the node codes: 24 rows 80 us per
 // step, 16 rows 85, 32 rows 98, 64 rows 92 (ring body 104).
 static int build_two(sclbm_batch *b, const int *tile_y)
 {
     if (b->prec == SCLBM_FP64) return SCLBM_OK;
-    for (auto *d : b->doms)
-        if (d->nx < 4 || d->ny < 4) return SCLBM_OK;
+    for (size_t k = 0; k < b->doms.size(); ++k)
+        if (b->doms[k]->nx < 4 || b->doms[k]->ny < 4 || (tile_y && !two_rows_pay(b->prec, std::max(0, tile_y[k]))))
+            return SCLBM_OK;
     auto bands_of = [&](const sclbm_domain *d, int k, int rows) {
         const int r = tile_y && tile_y[k] > 0 ? tile_y[k] : rows;
         return std::max(1, (int)((d->ny + r - 1) / r));

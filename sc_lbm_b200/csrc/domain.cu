@@ -491,12 +491,14 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
 // / 15.7), 1024^2 21.5 / 31.6; FP16 1024^2 24.6 / 24.0 (27.8 / 26.3), 1200^2 33 /
 // 33 (39 / 37), 2048 x 1024 44 / 47.5 (52 / 52).  Lattices that need 64-bit
 // offsets, and domains with a variant or a tile width of the caller's choice,
-// take single steps; a band height of the caller's choice asks for pairs.
+// take single steps; a band height of the caller's choice asks for pairs unless
+// it is too low for them.
 static bool two_step(const sclbm_domain *d)
 {
     const size_t most = d->prec == SCLBM_FP32_SHIFTED ? 450000 : 1500000;
     return d->variant == 0 && d->tx == 128 && d->ncomp == 2 && d->prec != SCLBM_FP64 && d->nx >= 4 &&
-           d->ny >= 4 && (d->tile_y > 0 || d->N > most) && !needs_wide_offsets(d->N);
+           d->ny >= 4 && (d->tile_y > 0 ? two_rows_pay(d->prec, d->tile_y) : d->N > most) &&
+           !needs_wide_offsets(d->N);
 }
 
 // two steps in one launch

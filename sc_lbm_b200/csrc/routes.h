@@ -28,6 +28,16 @@ inline bool flat_beats_tile(size_t nx, size_t ny, sclbm_precision p, bool solid)
     return n < 3 * M / 2 || (n < 3 * M && full < 0.985);
 }
 
+// Whether bands of a height of the caller's choice (0: none) run in pairs
+// (fused_two.cuh).  A band of r rows computes r + 4 rows of the first step, so low
+// ones lose to single steps of that height.  us per step, pairs / single steps:
+// FP32 2048^2 2 rows 151 / 121, 512^2 3 rows 11.2 / 10.4, 4 rows equal or faster; FP16
+// 2048^2 4 rows 115 / 103, 5 rows 104 / 100, 6 rows equal or faster.
+inline bool two_rows_pay(sclbm_precision p, int rows)
+{
+    return rows == 0 || rows >= (p == SCLBM_FP32_SHIFTED ? 4 : 6);
+}
+
 // ------------------------------------------------- single-component lattices
 // A launch of k_single (fused_single.cuh) takes as long as its tiles of 32 x 16
 // nodes with halo, however few nodes of their own they hold: 0.7 us and, per

@@ -23,6 +23,9 @@ int main()
         } else if (what == "flat") { // one node per thread rather than the register tile
             std::cin >> nx >> ny >> p >> keep;
             std::cout << flat_beats_tile(nx, ny, (sclbm_precision)p, keep != 0) << '\n';
+        } else if (what == "rows") { // bands of this height in pairs
+            std::cin >> p >> n;
+            std::cout << two_rows_pay((sclbm_precision)p, n) << '\n';
         } else {
             return 1;
         }

@@ -7,6 +7,17 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+def median_time(sclbm, call):
+    t = []
+    for _ in range(7):
+        sclbm.synchronize()
+        t0 = time.perf_counter()
+        call()
+        sclbm.synchronize()
+        t.append(time.perf_counter() - t0)
+    return np.median(t)
+
+
 @pytest.mark.parametrize("prec_name", ["FP64", "FP32_SHIFTED", "FP16_SHIFTED"])
 @pytest.mark.parametrize("nx", [1, 3, 4])
 def test_narrow_single_component_lattices(sclbm, prec_name, nx):
@@ -34,12 +45,35 @@ def test_narrow_single_component_lattices_cost_their_nodes(sclbm):
     def per_call(nx, ny):
         d = sclbm.Domain(nx, ny, np.ones(nx * ny, np.int32), sclbm.make_params(ncomp=1), sclbm.FP64)
         d.init_noise(0, 1.0, 0.01, 1)
-        t = []
-        for _ in range(7):
-            sclbm.synchronize()
-            t0 = time.perf_counter()
-            d.step(200)
-            sclbm.synchronize()
-            t.append(time.perf_counter() - t0)
-        return np.median(t)
+        return median_time(sclbm, lambda: d.step(200))
     assert per_call(4, 100000) < 3 * per_call(400, 1000)
+
+
+def pair_domain(sclbm, nx, ny, prec, variant, rows, seed=1):
+    from sc_lbm_b200 import workloads as W
+    mask = (W.uniform(2, nx * ny) < 0.8).astype(np.int32)
+    p = sclbm.make_params(ncomp=2, g_fluid=(0.9, 0.9), g_solid=(-0.1, 0.1))
+    d = sclbm.Domain(nx, ny, mask, p, prec)
+    d.set_kernel(variant, rows)
+    for k in range(2):
+        d.init_noise(k, 1.0, 0.1, seed + k)
+    return d
+
+
+@pytest.mark.parametrize("prec_name", ["FP32_SHIFTED", "FP16_SHIFTED"])
+@pytest.mark.parametrize("nx,ny,rows", [(4, 4, 6), (5, 7, 6), (64, 33, 6), (121, 13, 6), (122, 9, 8), (123, 6, 64),
+                                        (64, 33, 5), (64, 33, 4), (64, 33, 3)])
+def test_bands_on_both_sides_of_the_lowest_pair(sclbm, prec_name, nx, ny, rows):
+    prec = getattr(sclbm, prec_name)
+    a, b = (pair_domain(sclbm, nx, ny, prec, v, r) for v, r in ((0, rows), (2, 0)))
+    a.step(7)
+    b.step(7)
+    assert [a.download_f(k).tobytes() for k in range(2)] == [b.download_f(k).tobytes() for k in range(2)]
+
+
+def test_low_bands_cost_no_more_than_single_steps(sclbm):
+    """Bands of one row asked for: within half as much again as the register tile
+    (twice its time in pairs)."""
+    t = [median_time(sclbm, lambda d=d: d.step(100))
+         for d in (pair_domain(sclbm, 1024, 1024, sclbm.FP16_SHIFTED, v, r) for v, r in ((0, 1), (8, 0)))]
+    assert t[0] < 1.5 * t[1], t

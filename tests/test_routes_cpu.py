@@ -79,3 +79,11 @@ FLAT = [
 
 def test_single_steps_off_the_ring(ask):
     assert ask([("flat", *q) for q, _ in FLAT]) == [(int(want),) for _, want in FLAT]
+
+
+def test_low_bands_take_single_steps(ask):
+    """us per step, pairs / single steps: FP32 3 rows 11.2 / 10.4, 4 rows equal; FP16
+    5 rows 104 / 100, 6 rows equal."""
+    least = {FP32: 4, FP16: 6}
+    questions = [("rows", p, n) for p in least for n in (0, 1, 2, 3, 4, 5, 6, 7, 64)]
+    assert ask(questions) == [(int(n == 0 or n >= least[p]),) for _, p, n in questions]
