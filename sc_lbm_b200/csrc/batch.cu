@@ -250,8 +250,12 @@ static int build_two(sclbm_batch *b, const int *tile_y)
     }
     std::vector<TwoUnit> units;
     std::vector<long> cost;
+    double nodes = 0.0, strip_rows = 0.0;
     for (size_t k = 0; k < b->doms.size(); ++k) {
         const sclbm_domain *d = b->doms[k];
+        constexpr size_t W = TWO_TX - 6;
+        nodes += (double)d->N;
+        strip_rows += (double)((d->nx + W - 1) / W) * (double)d->ny;
         const int w = two_width((int)d->nx), bands = bands_of(d, (int)k, rows);
         for (int j = 0; j < bands; ++j) {
             const int y0 = (int)((long long)d->ny * j / bands), y1 = (int)((long long)d->ny * (j + 1) / bands);
@@ -261,6 +265,9 @@ static int build_two(sclbm_batch *b, const int *tile_y)
             }
         }
     }
+    if (b->body == BODY_WARP && !b->use_ring &&
+        !batch_two_beats_warp(strip_rows, nodes / (strip_rows * (TWO_TX - 6)), sm_count()))
+        return SCLBM_OK;
     // largest first at domain granularity, as the ring's units
     std::vector<long> dom_cost(b->doms.size(), 0);
     for (size_t i = 0; i < units.size(); ++i)

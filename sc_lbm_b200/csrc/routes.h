@@ -38,6 +38,16 @@ inline bool two_rows_pay(sclbm_precision p, int rows)
     return rows == 0 || rows >= (p == SCLBM_FP32_SHIFTED ? 4 : 6);
 }
 
+// Whether an FP16 batch with solid nodes, off the ring body, runs in pairs or in
+// the one-warp tiles that are its single-step body: strips of few columns leave
+// most of a pair kernel's CTA idle, which counts once the strips have more than
+// some 25 rows per SM.  rows: of all strips together; full: nodes over the columns
+// of whole strips.  us per step, pairs / one-warp tiles: 300 domains of 20 x 20 20.0
+// / 12.2 (41 rows per SM, full 0.16), 60 x 60 50 / 46 (122, 0.49), 90 x 60 57 / 71 (122,
+// 0.74), 12 x 8 9.4 / 9.7 (16, 0.10); 60 domains of 20 x 20 6.2 / 9.8 (8, 0.16), 44 x 60
+// 12.6 / 14.0 (24, 0.36).
+inline bool batch_two_beats_warp(double rows, double full, int sms) { return rows <= 25.0 * sms || full >= 0.6; }
+
 // ------------------------------------------------- single-component lattices
 // A launch of k_single (fused_single.cuh) takes as long as its tiles of 32 x 16
 // nodes with halo, however few nodes of their own they hold: 0.7 us and, per

@@ -26,6 +26,9 @@ int main()
         } else if (what == "rows") { // bands of this height in pairs
             std::cin >> p >> n;
             std::cout << two_rows_pay((sclbm_precision)p, n) << '\n';
+        } else if (what == "warp") { // rows of strips, thousandths of their columns, SMs
+            std::cin >> n >> K >> sms;
+            std::cout << batch_two_beats_warp(n, K / 1000.0, sms) << '\n';
         } else {
             return 1;
         }

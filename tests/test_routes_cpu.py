@@ -87,3 +87,11 @@ def test_low_bands_take_single_steps(ask):
     least = {FP32: 4, FP16: 6}
     questions = [("rows", p, n) for p in least for n in (0, 1, 2, 3, 4, 5, 6, 7, 64)]
     assert ask(questions) == [(int(n == 0 or n >= least[p]),) for _, p, n in questions]
+
+
+def test_narrow_fp16_domains_with_solid_nodes(ask):
+    """us per step of a batch, pairs / one-warp tiles: 300 x (20 x 20) 20.0 / 12.2,
+    300 x (60 x 60) 50 / 46, 300 x (90 x 60) 57 / 71, 300 x (12 x 8) 9.4 / 9.7, 60 x (20 x 20)
+    6.2 / 9.8, 60 x (44 x 60) 12.6 / 14.0."""
+    rows_full = [(6000, 163), (18000, 491), (18000, 737), (2400, 98), (1200, 163), (3600, 360)]
+    assert ask([("warp", *q, SMS) for q in rows_full]) == [(0,), (0,), (1,), (1,), (1,), (1,)]
