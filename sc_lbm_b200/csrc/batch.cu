@@ -285,20 +285,59 @@ static int build_two(sclbm_batch *b, const int *tile_y)
     return SCLBM_OK;
 }
 
-// Tiles of the one-node-per-thread kernel for FP64 batches.  With solid nodes
-// it is faster than the ring body (us per step: eight mixed domains 12.9 / 27.8,
-// eight 400 x 306 71 / 91, 64 mixed domains 211 / 225); without, as for a single
-// lattice, up to 4 M nodes.  Heights of the caller's choice ask for marching
-// tiles.
+// Turns from fluid to solid or back along the rows of a batch's masks; CTA rows
+// (blockIdx.y) take a domain each.
+__global__ void __launch_bounds__(256)
+    k_mask_changes(const Fused2Args<double, double> *__restrict__ doms, unsigned long long *__restrict__ sum)
+{
+    const uint8_t *mask = doms[2 * blockIdx.y].mask;
+    const size_t N = doms[2 * blockIdx.y].N;
+    unsigned n = 0;
+    for (size_t i = blockIdx.x * 256u + threadIdx.x; i + 1 < N; i += gridDim.x * 256u) n += mask[i] != mask[i + 1];
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(sum, n);
+}
+
+static int mask_changes(const sclbm_batch *b, double *out)
+{
+    cudaStream_t s = stream();
+    auto *sum = (unsigned long long *)b->doms[0]->partials; // scratch of the monitor
+    unsigned long long n = 0;
+    SCLBM_CUDA(cudaMemsetAsync(sum, 0, sizeof n, s));
+    for (size_t k = 0; k < b->doms.size(); k += 65535) {
+        const dim3 grid(16, (unsigned)std::min<size_t>(65535, b->doms.size() - k));
+        k_mask_changes<<<grid, 256, 0, s>>>((const Fused2Args<double, double> *)b->d_args + 2 * k, sum);
+        SCLBM_LAUNCHED("mask changes");
+    }
+    SCLBM_CUDA(cudaMemcpyAsync(&n, sum, sizeof n, cudaMemcpyDeviceToHost, s));
+    SCLBM_CUDA(cudaStreamSynchronize(s));
+    *out = (double)n;
+    return SCLBM_OK;
+}
+
+// Tiles of the one-node-per-thread kernel for FP64 batches: with solid nodes
+// where it is faster than the ring body (routes.h; eight mixed domains 12.9 / 27.8
+// us per step), without, as for a single lattice, up to 4 M nodes.  Heights of
+// the caller's choice ask for marching tiles.
 static int build_flat(sclbm_batch *b, const int *tile_y)
 {
     if (b->prec != SCLBM_FP64 || tile_y) return SCLBM_OK;
-    size_t nodes = 0, count = 0;
+    size_t nodes = 0, count = 0, strips = 0;
     for (auto *d : b->doms) {
         nodes += d->N;
+        if (const size_t w = (size_t)b->auto_ring) strips += (d->nx + w - 1) / w * w * d->ny;
         count += ((d->nx + 31) / 32) * ((d->ny + FLAT_ROWS - 1) / FLAT_ROWS);
     }
     if ((!(b->flags & KF_SOLID) && nodes >= ((size_t)1 << 22)) || count > ((size_t)1 << 30)) return SCLBM_OK;
+    if ((b->flags & KF_SOLID) && b->auto_ring) {
+        const double full = (double)nodes / (double)strips;
+        double changes = 0.0; // counted where they decide
+        if (batch_flat_beats_ring((double)nodes, full, 0.0) != batch_flat_beats_ring((double)nodes, full, 1.0)) {
+            const int rc = mask_changes(b, &changes);
+            if (rc) return rc;
+        }
+        if (!batch_flat_beats_ring((double)nodes, full, changes / (double)nodes)) return SCLBM_OK;
+    }
     std::vector<FlatTile> tiles;
     tiles.reserve(count);
     for (size_t k = 0; k < b->doms.size(); ++k)

@@ -48,6 +48,22 @@ inline bool two_rows_pay(sclbm_precision p, int rows)
 // 12.6 / 14.0 (24, 0.36).
 inline bool batch_two_beats_warp(double rows, double full, int sms) { return rows <= 25.0 * sms || full >= 0.6; }
 
+// FP64 batches with solid nodes that the ring body takes: one node per thread, or
+// the ring.  full: nodes over the columns of whole ring strips (which the ring
+// computes in vain); changes: how often a row turns from fluid to solid or back,
+// per node (the scattered stores of one node per thread).  us per step, one node
+// per thread / ring: 2 x 1024^2 with disks of radius 10-30 (0.027) 139 / 155, 4-16
+// (0.052) 155 / 163, 2-4 (0.079) 179 / 173, 10 % of all nodes solid (0.18) 198 / 183;
+// 24 x (400 x 306), strips 78 % full, (0.027) 203 / 257, (0.18) 272 / 285; 16 x 512^2
+// (0.056) 309 / 301; 200 x (320 x 160) 769 / 784; 4 x 256^2 (0.18) 20 / 28.
+inline bool batch_flat_beats_ring(double nodes, double full, double changes)
+{
+    if (nodes < 1e6) return true;
+    const bool loose = full < 0.9;
+    if (nodes < 4e6) return changes < (loose ? 0.15 : 0.06);
+    return nodes < 8e6 && loose && changes < 0.06;
+}
+
 // ------------------------------------------------- single-component lattices
 // A launch of k_single (fused_single.cuh) takes as long as its tiles of 32 x 16
 // nodes with halo, however few nodes of their own they hold: 0.7 us and, per

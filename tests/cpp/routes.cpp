@@ -29,6 +29,9 @@ int main()
         } else if (what == "warp") { // rows of strips, thousandths of their columns, SMs
             std::cin >> n >> K >> sms;
             std::cout << batch_two_beats_warp(n, K / 1000.0, sms) << '\n';
+        } else if (what == "batch64") { // thousands of nodes, thousandths full, changes per 1000 nodes
+            std::cin >> nx >> K >> n;
+            std::cout << batch_flat_beats_ring(1000.0 * (double)nx, K / 1000.0, n / 1000.0) << '\n';
         } else {
             return 1;
         }

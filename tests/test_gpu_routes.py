@@ -93,3 +93,54 @@ def test_many_narrow_domains_keep_their_one_warp_tiles(sclbm):
     t = [median_time(sclbm, lambda x=x: x.step(200)) for x in (x, y)]
     assert t[0] < 1.3 * t[1], t
     assert all(p.download_f(0).tobytes() == q.download_f(0).tobytes() for p, q in zip(a[::37], b[::37]))
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("porous", [False, True])
+def test_fp64_batch_of_ragged_lattices(sclbm, graph, porous):
+    """One node per thread on heights off its tiles' four rows and widths off 32."""
+    from sc_lbm_b200 import workloads as W
+    sizes = [(1, 9), (7, 1), (33, 5), (129, 130), (31, 3), (1, 1), (64, 37)]
+    doms, alone = [], []
+    for out, variant in ((doms, 0), (alone, 2)):
+        for k, (nx, ny) in enumerate(sizes):
+            n = nx * ny
+            mask = (W.uniform(k, n) < 0.75).astype(np.int32) if porous else np.ones(n, np.int32)
+            F = (W.force_vec(1e-4, "x"), W.force_vec(2e-4, "y")) if k % 2 else (None, None)
+            d = sclbm.Domain(nx, ny, mask, sclbm.make_params(g_fluid=(0.9, 0.9), g_solid=(-0.1, 0.1), force=F),
+                             sclbm.FP64)
+            d.set_kernel(variant)
+            for c in range(2):
+                d.upload_f(c, W.populations(1 + 0.1 * (2 * W.uniform(5 + c + k, n) - 1), mask))
+            out.append(d)
+    batch = sclbm.Batch(doms)
+    batch.step(23, graph)
+    for d, a, size in zip(doms, alone, sizes):
+        a.step(23)
+        for c in range(2):
+            assert d.download_f(c).tobytes() == a.download_f(c).tobytes(), size
+
+
+@pytest.mark.parametrize("radii,flat", [((10, 30), True), (None, False)])
+def test_fp64_batch_of_scattered_solids(sclbm, radii, flat):
+    """Large disks: one node per thread; every tenth node solid: the ring."""
+    from sc_lbm_b200 import workloads as W
+    nx, ny, n = 1024, 512, 1024 * 512
+    mask = np.ones(n, np.int32) if radii else (W.uniform(1, n) < 0.9).astype(np.int32)
+    p = sclbm.make_params(g_fluid=(0.9, 0.9), g_solid=(-0.1, 0.1))
+    doms = [sclbm.Domain(nx, ny, mask, p, sclbm.FP64) for _ in range(3)]
+    for d in doms:
+        if radii:
+            d.add_random_disks(0.7, *radii, 3)
+        for c in range(2):
+            d.init_noise(c, 1.0, 0.1, 3 + c)
+    batch = sclbm.Batch(doms)
+    tiles = 3 * (nx // 32) * (ny // 4)
+    assert (batch.info()[0] == tiles) == flat
+    batch.step(3)
+    one = sclbm.Domain(nx, ny, doms[0].download_mask(), p, sclbm.FP64)
+    one.set_kernel(2)
+    for c in range(2):
+        one.init_noise(c, 1.0, 0.1, 3 + c)
+    one.step(3)
+    assert all(d.download_f(0).tobytes() == one.download_f(0).tobytes() for d in doms)

@@ -95,3 +95,21 @@ def test_narrow_fp16_domains_with_solid_nodes(ask):
     6.2 / 9.8, 60 x (44 x 60) 12.6 / 14.0."""
     rows_full = [(6000, 163), (18000, 491), (18000, 737), (2400, 98), (1200, 163), (3600, 360)]
     assert ask([("warp", *q, SMS) for q in rows_full]) == [(0,), (0,), (1,), (1,), (1,), (1,)]
+
+
+# thousand nodes, fill of the ring's strips and changes along rows in
+# thousandths: whether one node per thread was faster than the ring (us per step)
+BATCH64 = [
+    ((262, 1000, 180), True),                             # 4 x 256^2 20 / 28
+    ((979, 781, 180), True),                              # 8 x (400 x 306) 94 / 100
+    ((1311, 1000, 56), True), ((1311, 1000, 95), False),  # 5 x 512^2 100 / 106; 115 / 113
+    ((2097, 1000, 52), True), ((2097, 1000, 79), False),  # 2 x 1024^2 155 / 163; 179 / 173
+    ((2938, 781, 118), True),                             # 24 x (400 x 306) 255 / 276
+    ((3840, 781, 94), True), ((3840, 781, 180), False),   # 64 x (300 x 200) 337 / 345; 377 / 362
+    ((4194, 1000, 56), False),                            # 16 x 512^2 309 / 301
+    ((4896, 781, 45), True), ((10240, 833, 55), False),   # 40 x (400 x 306) 369 / 401; the 512-domain ensemble 1685 / 1673
+]
+
+
+def test_fp64_batches_with_solid_nodes(ask):
+    assert ask([("batch64", *q) for q, _ in BATCH64]) == [(int(want),) for _, want in BATCH64]
