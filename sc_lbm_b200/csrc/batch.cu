@@ -14,7 +14,9 @@
 // The automatic choice and the rows per tile come from the autotuned size-class
 // table (tuning.h), weighted by the nodes of each class in the batch.
 #include <algorithm>
+#include <memory>
 #include <numeric>
+#include <utility>
 
 #include "domain.h"
 #include "batch_kernel.cuh"
@@ -33,6 +35,7 @@ static constexpr int GRAPH_STEPS = 20; // steps per captured graph (a multiple o
 struct sclbm_batch {
     std::vector<sclbm_domain *> doms;
     sclbm_precision prec = SCLBM_FP32_SHIFTED;
+    void *d_lists = nullptr; // the allocation that holds all device lists
     void *d_args = nullptr;  // Fused2Args<S,T>[2*ndom] (parity 0, parity 1)
     TileRef *d_tiles = nullptr;
     TileRef *d_tiles_half = nullptr; // 64-column tiles of the two-tiles-per-CTA body
@@ -70,6 +73,40 @@ struct sclbm_batch {
     FlatTile *d_flat = nullptr;
     int nflat = 0;
     bool use_flat = false;
+};
+
+// Device lists of a batch: one allocation, filled by copies in the stream that
+// the batch's kernels run in, all of them done when send returns (a cudaMemcpy
+// of pageable memory may return before its data has arrived, and does not order
+// other streams).  The lists stay on the host until then.
+struct DeviceLists {
+    struct Part {
+        void **list;
+        std::shared_ptr<void> keep;
+        const void *data;
+        size_t bytes, at;
+    };
+    std::vector<Part> parts;
+    size_t bytes = 0;
+
+    template <typename P, typename T> void add(P **list, std::vector<T> v)
+    {
+        auto keep = std::make_shared<std::vector<T>>(std::move(v));
+        const size_t n = keep->size() * sizeof(T), at = (bytes + 255) / 256 * 256;
+        parts.push_back(Part{(void **)list, keep, keep->data(), n, at});
+        bytes = at + n;
+    }
+    int send(void **base)
+    {
+        cudaStream_t s = stream();
+        SCLBM_CUDA(cudaMalloc(base, std::max<size_t>(bytes, 16)));
+        for (auto &p : parts) {
+            *p.list = (char *)*base + p.at;
+            if (p.bytes) SCLBM_CUDA(cudaMemcpyAsync(*p.list, p.data, p.bytes, cudaMemcpyHostToDevice, s));
+        }
+        SCLBM_CUDA(cudaStreamSynchronize(s));
+        return SCLBM_OK;
+    }
 };
 
 // the tile list of the current body
@@ -128,7 +165,7 @@ static cudaError_t batch_launch_any(sclbm_batch *b, int parity, cudaStream_t s)
 // largest units first; tensor maps of both parities of every domain.
 template <typename S, typename T>
 static int build_ring(sclbm_batch *b, const std::vector<Fused2Args<S, T>> &h, const std::vector<int> &rows,
-                      int width)
+                      int width, DeviceLists &lists)
 {
     const int r = width == 64 ? 1 : 0;
     std::vector<RingUnit> units;
@@ -166,25 +203,22 @@ static int build_ring(sclbm_batch *b, const std::vector<Fused2Args<S, T>> &h, co
     if (rc) return rc;
     b->nunits[r] = (int)sorted.size();
     b->ring_grid[r] = std::max(1, std::min(b->nunits[r], std::max(1, per_sm) * sm_count()));
-    SCLBM_CUDA(cudaMalloc(&b->d_units[r], sorted.size() * sizeof(RingUnit)));
-    SCLBM_CUDA(cudaMemcpy(b->d_units[r], sorted.data(), sorted.size() * sizeof(RingUnit),
-                          cudaMemcpyHostToDevice));
-    SCLBM_CUDA(cudaMalloc(&b->d_maps[r], maps.size() * sizeof(RingMaps)));
-    SCLBM_CUDA(cudaMemcpy(b->d_maps[r], maps.data(), maps.size() * sizeof(RingMaps), cudaMemcpyHostToDevice));
+    lists.add(&b->d_units[r], std::move(sorted));
+    lists.add(&b->d_maps[r], std::move(maps));
     return SCLBM_OK;
 }
 
 template <typename S, typename T>
-static int build_rings(sclbm_batch *b, const std::vector<Fused2Args<S, T>> &h, const std::vector<int> &rows)
+static int build_rings(sclbm_batch *b, const std::vector<Fused2Args<S, T>> &h, const std::vector<int> &rows,
+                       DeviceLists &lists)
 {
     const int A = 16 / (int)sizeof(S);
     for (auto *d : b->doms)
         if (d->nx % A != 0) return SCLBM_OK; // no ring body for this batch
-    int rc = build_ring<S, T>(b, h, rows, 128);
-    if (!rc) rc = build_ring<S, T>(b, h, rows, 64);
+    int rc = build_ring<S, T>(b, h, rows, 128, lists);
+    if (!rc) rc = build_ring<S, T>(b, h, rows, 64, lists);
     if (rc) return rc;
-    SCLBM_CUDA(cudaMalloc(&b->d_counters, 2 * sizeof(unsigned)));
-    SCLBM_CUDA(cudaMemset(b->d_counters, 0, 2 * sizeof(unsigned)));
+    lists.add(&b->d_counters, std::vector<unsigned>(2, 0u));
     b->ring = true;
     return SCLBM_OK;
 }
@@ -194,7 +228,8 @@ static int build_rings(sclbm_batch *b, const std::vector<Fused2Args<S, T>> &h, c
 constexpr int RING_BATCH_ROWS = 32;
 
 template <typename S, typename T>
-static int upload_args(sclbm_batch *b, const std::vector<int> &ty, const std::vector<int> &ring_rows)
+static int build_args(sclbm_batch *b, const std::vector<int> &ty, const std::vector<int> &ring_rows,
+                      DeviceLists &lists)
 {
     std::vector<Fused2Args<S, T>> h(2 * b->doms.size());
     for (size_t k = 0; k < b->doms.size(); ++k) {
@@ -214,34 +249,35 @@ static int upload_args(sclbm_batch *b, const std::vector<int> &ty, const std::ve
         d->parity = par;
         d->tile_y = saved_ty;
     }
-    SCLBM_CUDA(cudaMalloc(&b->d_args, h.size() * sizeof(Fused2Args<S, T>)));
-    SCLBM_CUDA(cudaMemcpy(b->d_args, h.data(), h.size() * sizeof(Fused2Args<S, T>),
-                          cudaMemcpyHostToDevice));
-    return build_rings<S, T>(b, h, ring_rows);
+    const int rc = build_rings<S, T>(b, h, ring_rows, lists);
+    lists.add(&b->d_args, std::move(h));
+    return rc;
 }
 
 // Units of the two-step kernel: per domain its strips and bands, all of about
 // the rows that two_cost finds best for the batch's units (the caller's height
 // where given; none when one of those is too low for pairs).  64 mixed domains, before the node codes: 24 rows 80 us per
 // step, 16 rows 85, 32 rows 98, 64 rows 92 (ring body 104).
-static int build_two(sclbm_batch *b, const int *tile_y)
+static void build_two(sclbm_batch *b, const int *tile_y, DeviceLists &lists)
 {
-    if (b->prec == SCLBM_FP64) return SCLBM_OK;
+    if (b->prec == SCLBM_FP64) return;
     for (size_t k = 0; k < b->doms.size(); ++k)
         if (b->doms[k]->nx < 4 || b->doms[k]->ny < 4 || (tile_y && !two_rows_pay(b->prec, std::max(0, tile_y[k]))))
-            return SCLBM_OK;
+            return;
     auto bands_of = [&](const sclbm_domain *d, int k, int rows) {
         const int r = tile_y && tile_y[k] > 0 ? tile_y[k] : rows;
         return std::max(1, (int)((d->ny + r - 1) / r));
     };
+    std::vector<int> width(b->doms.size()), strips(b->doms.size());
+    for (size_t k = 0; k < b->doms.size(); ++k) {
+        width[k] = two_width((int)b->doms[k]->nx);
+        strips[k] = ((int)b->doms[k]->nx + width[k] - 1) / width[k];
+    }
     int rows = 1;
     double least = 0.0;
     for (int r : TWO_ROWS) {
         long n = 0;
-        for (size_t k = 0; k < b->doms.size(); ++k) {
-            const int nx = (int)b->doms[k]->nx, w = two_width(nx);
-            n += (long)((nx + w - 1) / w) * bands_of(b->doms[k], (int)k, r);
-        }
+        for (size_t k = 0; k < b->doms.size(); ++k) n += (long)strips[k] * bands_of(b->doms[k], (int)k, r);
         const double cost = two_cost(n, r, sm_count());
         if (least == 0.0 || cost < least) {
             least = cost;
@@ -256,7 +292,7 @@ static int build_two(sclbm_batch *b, const int *tile_y)
         constexpr size_t W = TWO_TX - 6;
         nodes += (double)d->N;
         strip_rows += (double)((d->nx + W - 1) / W) * (double)d->ny;
-        const int w = two_width((int)d->nx), bands = bands_of(d, (int)k, rows);
+        const int w = width[k], bands = bands_of(d, (int)k, rows);
         for (int j = 0; j < bands; ++j) {
             const int y0 = (int)((long long)d->ny * j / bands), y1 = (int)((long long)d->ny * (j + 1) / bands);
             for (int xb = 0; xb < (int)d->nx; xb += w) {
@@ -267,7 +303,7 @@ static int build_two(sclbm_batch *b, const int *tile_y)
     }
     if (b->body == BODY_WARP && !b->use_ring &&
         !batch_two_beats_warp(strip_rows, nodes / (strip_rows * (TWO_TX - 6)), sm_count()))
-        return SCLBM_OK;
+        return;
     // largest first at domain granularity, as the ring's units
     std::vector<long> dom_cost(b->doms.size(), 0);
     for (size_t i = 0; i < units.size(); ++i)
@@ -278,22 +314,25 @@ static int build_two(sclbm_batch *b, const int *tile_y)
                      [&](int x, int y) { return dom_cost[units[x].dom] > dom_cost[units[y].dom]; });
     std::vector<TwoUnit> sorted(units.size());
     for (size_t i = 0; i < order.size(); ++i) sorted[i] = units[order[i]];
-    SCLBM_CUDA(cudaMalloc(&b->d_two, sorted.size() * sizeof(TwoUnit)));
-    SCLBM_CUDA(cudaMemcpy(b->d_two, sorted.data(), sorted.size() * sizeof(TwoUnit), cudaMemcpyHostToDevice));
     b->ntwo = (int)sorted.size();
+    lists.add(&b->d_two, std::move(sorted));
     b->use_two = true;
-    return SCLBM_OK;
 }
 
-// Turns from fluid to solid or back along the rows of a batch's masks; CTA rows
-// (blockIdx.y) take a domain each.
+// Turns from fluid to solid or back along the rows of some masks; CTA rows
+// (blockIdx.y) take one each.
+struct MaskGroup {
+    static constexpr int MOST = 128;
+    const uint8_t *mask[MOST];
+    uint32_t N[MOST]; // a batch's domains have fewer than 2^32 / 9 nodes
+};
 __global__ void __launch_bounds__(256)
-    k_mask_changes(const Fused2Args<double, double> *__restrict__ doms, unsigned long long *__restrict__ sum)
+    k_mask_changes(const __grid_constant__ MaskGroup g, unsigned long long *__restrict__ sum)
 {
-    const uint8_t *mask = doms[2 * blockIdx.y].mask;
-    const size_t N = doms[2 * blockIdx.y].N;
+    const uint8_t *mask = g.mask[blockIdx.y];
+    const uint32_t N = g.N[blockIdx.y];
     unsigned n = 0;
-    for (size_t i = blockIdx.x * 256u + threadIdx.x; i + 1 < N; i += gridDim.x * 256u) n += mask[i] != mask[i + 1];
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i + 1 < N; i += gridDim.x * 256) n += mask[i] != mask[i + 1];
     n = __reduce_add_sync(0xffffffffu, n);
     if ((threadIdx.x & 31) == 0 && n) atomicAdd(sum, n);
 }
@@ -304,9 +343,14 @@ static int mask_changes(const sclbm_batch *b, double *out)
     auto *sum = (unsigned long long *)b->doms[0]->partials; // scratch of the monitor
     unsigned long long n = 0;
     SCLBM_CUDA(cudaMemsetAsync(sum, 0, sizeof n, s));
-    for (size_t k = 0; k < b->doms.size(); k += 65535) {
-        const dim3 grid(16, (unsigned)std::min<size_t>(65535, b->doms.size() - k));
-        k_mask_changes<<<grid, 256, 0, s>>>((const Fused2Args<double, double> *)b->d_args + 2 * k, sum);
+    for (size_t k = 0; k < b->doms.size(); k += MaskGroup::MOST) {
+        MaskGroup g;
+        const int n_g = (int)std::min<size_t>(MaskGroup::MOST, b->doms.size() - k);
+        for (int j = 0; j < n_g; ++j) {
+            g.mask[j] = b->doms[k + j]->d_mask;
+            g.N[j] = (uint32_t)b->doms[k + j]->N;
+        }
+        k_mask_changes<<<dim3(16, n_g), 256, 0, s>>>(g, sum);
         SCLBM_LAUNCHED("mask changes");
     }
     SCLBM_CUDA(cudaMemcpyAsync(&n, sum, sizeof n, cudaMemcpyDeviceToHost, s));
@@ -319,7 +363,7 @@ static int mask_changes(const sclbm_batch *b, double *out)
 // where it is faster than the ring body (routes.h; eight mixed domains 12.9 / 27.8
 // us per step), without, as for a single lattice, up to 4 M nodes.  Heights of
 // the caller's choice ask for marching tiles.
-static int build_flat(sclbm_batch *b, const int *tile_y)
+static int build_flat(sclbm_batch *b, const int *tile_y, DeviceLists &lists)
 {
     if (b->prec != SCLBM_FP64 || tile_y) return SCLBM_OK;
     size_t nodes = 0, count = 0, strips = 0;
@@ -343,9 +387,8 @@ static int build_flat(sclbm_batch *b, const int *tile_y)
     for (size_t k = 0; k < b->doms.size(); ++k)
         for (size_t y = 0; y < b->doms[k]->ny; y += FLAT_ROWS)
             for (size_t x = 0; x < b->doms[k]->nx; x += 32) tiles.push_back(FlatTile{(int)k, (int)x, (int)y});
-    SCLBM_CUDA(cudaMalloc(&b->d_flat, tiles.size() * sizeof(FlatTile)));
-    SCLBM_CUDA(cudaMemcpy(b->d_flat, tiles.data(), tiles.size() * sizeof(FlatTile), cudaMemcpyHostToDevice));
     b->nflat = (int)tiles.size();
+    lists.add(&b->d_flat, std::move(tiles));
     b->use_flat = true;
     return SCLBM_OK;
 }
@@ -366,18 +409,7 @@ void sclbm_batch_destroy(sclbm_batch *b)
     if (!b) return;
     for (auto &g : b->graph)
         if (g) cudaGraphExecDestroy(g);
-    if (b->d_args) cudaFree(b->d_args);
-    if (b->d_tiles) cudaFree(b->d_tiles);
-    if (b->d_tiles_half) cudaFree(b->d_tiles_half);
-    if (b->d_tiles_warp) cudaFree(b->d_tiles_warp);
-    if (b->d_bands) cudaFree(b->d_bands);
-    for (int r = 0; r < 2; ++r) {
-        if (b->d_units[r]) cudaFree(b->d_units[r]);
-        if (b->d_maps[r]) cudaFree(b->d_maps[r]);
-    }
-    if (b->d_counters) cudaFree(b->d_counters);
-    if (b->d_two) cudaFree(b->d_two);
-    if (b->d_flat) cudaFree(b->d_flat);
+    if (b->d_lists) cudaFree(b->d_lists);
     delete b;
 }
 
@@ -465,9 +497,9 @@ int sclbm_batch_create(sclbm_domain *const *domains, int ndomains, const int *ti
         for (size_t i = 0; i < order.size(); ++i) sorted[i] = list[order[i]];
         return sorted;
     };
-    const std::vector<TileRef> sorted = tile_list(BATCH_TX);
-    const std::vector<TileRef> halves = tile_list(HALF_TX);
-    const std::vector<TileRef> warps = tile_list(WARP_TX);
+    std::vector<TileRef> sorted = tile_list(BATCH_TX);
+    std::vector<TileRef> halves = tile_list(HALF_TX);
+    std::vector<TileRef> warps = tile_list(WARP_TX);
     b->ntiles = (int)sorted.size();
     b->ntiles_half = (int)halves.size();
     b->ntiles_warp = (int)warps.size();
@@ -508,10 +540,11 @@ int sclbm_batch_create(sclbm_domain *const *domains, int ndomains, const int *ti
             if (!changed) break;
         }
     }
+    DeviceLists lists;
     switch (b->prec) {
-    case SCLBM_FP64: rc = upload_args<double, double>(b, ty, ring_rows); break;
-    case SCLBM_FP32_SHIFTED: rc = upload_args<float, float>(b, ty, ring_rows); break;
-    default: rc = upload_args<__half, float>(b, ty, ring_rows); break;
+    case SCLBM_FP64: rc = build_args<double, double>(b, ty, ring_rows, lists); break;
+    case SCLBM_FP32_SHIFTED: rc = build_args<float, float>(b, ty, ring_rows, lists); break;
+    default: rc = build_args<__half, float>(b, ty, ring_rows, lists); break;
     }
     // pipelined kernel: the smallest band height whose (domain, strip, band)
     // tiles all fit resident at once, bands of one domain split its rows evenly.
@@ -572,29 +605,14 @@ int sclbm_batch_create(sclbm_domain *const *domains, int ndomains, const int *ti
         }
         b->nbands = (int)bands.size();
         b->band_grid = std::max(1, std::min(b->nbands, res));
-        if (!rc && cudaMalloc(&b->d_bands, bands.size() * sizeof(BandTile)) != cudaSuccess)
-            rc = set_error(SCLBM_E_CUDA, "band list allocation");
-        if (!rc && cudaMemcpy(b->d_bands, bands.data(), bands.size() * sizeof(BandTile),
-                              cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = set_error(SCLBM_E_CUDA, "band list upload");
+        lists.add(&b->d_bands, std::move(bands));
     }
-    if (!rc && cudaMalloc(&b->d_tiles, sorted.size() * sizeof(TileRef)) != cudaSuccess)
-        rc = set_error(SCLBM_E_CUDA, "tile list allocation");
-    if (!rc && cudaMemcpy(b->d_tiles, sorted.data(), sorted.size() * sizeof(TileRef),
-                          cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = set_error(SCLBM_E_CUDA, "tile list upload");
-    if (!rc && cudaMalloc(&b->d_tiles_warp, warps.size() * sizeof(TileRef)) != cudaSuccess)
-        rc = set_error(SCLBM_E_CUDA, "tile list allocation");
-    if (!rc && cudaMemcpy(b->d_tiles_warp, warps.data(), warps.size() * sizeof(TileRef),
-                          cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = set_error(SCLBM_E_CUDA, "tile list upload");
-    if (!rc && cudaMalloc(&b->d_tiles_half, halves.size() * sizeof(TileRef)) != cudaSuccess)
-        rc = set_error(SCLBM_E_CUDA, "tile list allocation");
-    if (!rc && cudaMemcpy(b->d_tiles_half, halves.data(), halves.size() * sizeof(TileRef),
-                          cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = set_error(SCLBM_E_CUDA, "tile list upload");
-    if (!rc) rc = build_two(b, tile_y_per_domain);
-    if (!rc) rc = build_flat(b, tile_y_per_domain);
+    lists.add(&b->d_tiles, std::move(sorted));
+    lists.add(&b->d_tiles_warp, std::move(warps));
+    lists.add(&b->d_tiles_half, std::move(halves));
+    if (!rc) build_two(b, tile_y_per_domain, lists);
+    if (!rc) rc = build_flat(b, tile_y_per_domain, lists);
+    if (!rc) rc = lists.send(&b->d_lists);
     if (rc) {
         sclbm_batch_destroy(b);
         return rc;
