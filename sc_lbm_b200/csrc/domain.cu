@@ -610,7 +610,6 @@ void sclbm_domain_destroy(sclbm_domain *d)
     for (auto *p : d->rho_tmp)
         if (p) cudaFree(p);
     if (d->d_mask) cudaFree(d->d_mask);
-    if (d->d_codes) cudaFree(d->d_codes);
     if (d->staging) cudaFree(d->staging);
     if (d->partials) cudaFree(d->partials);
     if (d->d_status) cudaFree(d->d_status);
@@ -650,8 +649,16 @@ int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_p
     d->p = *p;
     if (precision == SCLBM_FP64) d->p.rho_ref[0] = d->p.rho_ref[1] = 0.0;
     const size_t es = elem_size(precision);
+    const bool coded = precision != SCLBM_FP64 && d->ncomp == 2;
+    const size_t codes_at = (N + 15) & ~size_t(15), codes = (N * sizeof(uint16_t) + 15) & ~size_t(15);
     cudaStream_t s = stream();
-    if ((rc = dom_alloc(d, (void **)&d->d_mask, N))) goto fail;
+    // the mask; behind it, where the kernels use them, the node codes and their
+    // sums (an allocation of their own made creation 10 % dearer)
+    if ((rc = dom_alloc(d, (void **)&d->d_mask, coded ? codes_at + codes + 256 * sizeof(float2) : N))) goto fail;
+    if (coded) {
+        d->d_codes = (uint16_t *)(d->d_mask + codes_at);
+        d->d_sums = (float2 *)(d->d_mask + codes_at + codes);
+    }
     for (int par = 0; par < 2; ++par)
         for (int k = 0; k < d->ncomp; ++k) {
             if ((rc = dom_alloc(d, &d->buf[par][k], 9 * N * es))) goto fail;
@@ -674,11 +681,6 @@ int sclbm_domain_create(size_t nx, size_t ny, const int32_t *mask, const sclbm_p
     if (cudaMemsetAsync(d->d_status, 0, sizeof(int), s) != cudaSuccess) {
         rc = set_error(SCLBM_E_CUDA, "memset");
         goto fail;
-    }
-    if (precision != SCLBM_FP64 && d->ncomp == 2) {
-        const size_t codes = (N * sizeof(uint16_t) + 15) & ~size_t(15);
-        if ((rc = dom_alloc(d, (void **)&d->d_codes, codes + 256 * sizeof(float2)))) goto fail;
-        d->d_sums = (float2 *)((char *)d->d_codes + codes);
     }
     if (cudaMemcpyAsync(d->d_mask, hm.data(), N, cudaMemcpyHostToDevice, s) != cudaSuccess ||
         domain_refresh_codes(d, s) != SCLBM_OK || cudaStreamSynchronize(s) != cudaSuccess) {

@@ -8,8 +8,8 @@ struct sclbm_domain {
     sclbm_precision prec = SCLBM_FP64;
     sclbm_params p{};
     uint8_t *d_mask = nullptr;
-    uint16_t *d_codes = nullptr; // node codes of the mask (two-component shifted forms), and
-    float2 *d_sums = nullptr;    // behind them the sums by neighbour bits
+    uint16_t *d_codes = nullptr; // behind the mask: its node codes (two-component shifted forms)
+    float2 *d_sums = nullptr;    // and the sums by neighbour bits
     void *buf[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}}; // [parity][comp], 9N each
     int parity = 0; // buf[parity] holds the state; turns over with every step
     void *rho_tmp[2] = {nullptr, nullptr}; // density arrays of the two-pass variant
