@@ -261,9 +261,8 @@ static int build_args(sclbm_batch *b, const std::vector<int> &ty, const std::vec
 static void build_two(sclbm_batch *b, const int *tile_y, DeviceLists &lists)
 {
     if (b->prec == SCLBM_FP64) return;
-    for (size_t k = 0; k < b->doms.size(); ++k)
-        if (b->doms[k]->nx < 4 || b->doms[k]->ny < 4 || (tile_y && !two_rows_pay(b->prec, std::max(0, tile_y[k]))))
-            return;
+    for (auto *d : b->doms)
+        if (d->nx < 4 || d->ny < 4) return;
     auto bands_of = [&](const sclbm_domain *d, int k, int rows) {
         const int r = tile_y && tile_y[k] > 0 ? tile_y[k] : rows;
         return std::max(1, (int)((d->ny + r - 1) / r));
@@ -284,12 +283,18 @@ static void build_two(sclbm_batch *b, const int *tile_y, DeviceLists &lists)
             rows = r;
         }
     }
+    if (tile_y) {
+        long n = 0;
+        for (size_t k = 0; k < b->doms.size(); ++k) n += (long)strips[k] * bands_of(b->doms[k], (int)k, rows);
+        for (size_t k = 0; k < b->doms.size(); ++k)
+            if (!two_rows_pay(b->prec, std::max(0, tile_y[k]), n, b->flags & KF_SOLID, sm_count())) return;
+    }
     std::vector<TwoUnit> units;
     std::vector<long> cost;
     double nodes = 0.0, strip_rows = 0.0;
     for (size_t k = 0; k < b->doms.size(); ++k) {
         const sclbm_domain *d = b->doms[k];
-        constexpr size_t W = TWO_TX - 6;
+        constexpr size_t W = TWO_COLUMNS;
         nodes += (double)d->N;
         strip_rows += (double)((d->nx + W - 1) / W) * (double)d->ny;
         const int w = width[k], bands = bands_of(d, (int)k, rows);
@@ -302,7 +307,7 @@ static void build_two(sclbm_batch *b, const int *tile_y, DeviceLists &lists)
         }
     }
     if (b->body == BODY_WARP && !b->use_ring &&
-        !batch_two_beats_warp(strip_rows, nodes / (strip_rows * (TWO_TX - 6)), sm_count()))
+        !batch_two_beats_warp(strip_rows, nodes / (strip_rows * TWO_COLUMNS), sm_count()))
         return;
     // largest first at domain granularity, as the ring's units
     std::vector<long> dom_cost(b->doms.size(), 0);

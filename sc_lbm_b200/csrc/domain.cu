@@ -495,10 +495,12 @@ static cudaError_t step_one(const sclbm_domain *d, cudaStream_t s)
 // it is too low for them.
 static bool two_step(const sclbm_domain *d)
 {
-    const size_t most = d->prec == SCLBM_FP32_SHIFTED ? 450000 : 1500000;
-    return d->variant == 0 && d->tx == 128 && d->ncomp == 2 && d->prec != SCLBM_FP64 && d->nx >= 4 &&
-           d->ny >= 4 && (d->tile_y > 0 ? two_rows_pay(d->prec, d->tile_y) : d->N > most) &&
-           !needs_wide_offsets(d->N);
+    if (d->variant != 0 || d->tx != 128 || d->ncomp != 2 || d->prec == SCLBM_FP64 || d->nx < 4 || d->ny < 4 ||
+        needs_wide_offsets(d->N))
+        return false;
+    if (d->tile_y == 0) return d->N > (d->prec == SCLBM_FP32_SHIFTED ? 450000 : 1500000);
+    const long units = (long)((d->nx + TWO_COLUMNS - 1) / TWO_COLUMNS) * (long)((d->ny + d->tile_y - 1) / d->tile_y);
+    return two_rows_pay(d->prec, d->tile_y, units, d->has_solid, sm_count());
 }
 
 // two steps in one launch

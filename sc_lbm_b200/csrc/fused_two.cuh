@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(TX, TWO_CTAS)
 // on five warps, 64 + 64 on six.
 inline int two_width(int nx)
 {
-    constexpr int W = TWO_TX - 6;
+    constexpr int W = TWO_COLUMNS;
+    static_assert(W == TWO_TX - 6, "a strip's columns and three more on each side");
     const int strips = (nx + W - 1) / W, even = (nx + strips - 1) / strips;
     int best = even, least = 0;
     for (int w = even; w <= W; ++w) {

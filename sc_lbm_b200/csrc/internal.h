@@ -227,6 +227,7 @@ cudaError_t launch_single_f16(const Fused1Args<__half, float> &a, int K, int ste
 // the state two steps later; rows per band (0 default)
 cudaError_t launch_two2_f32(const Fused2Args<float, float> &a, int rows, cudaStream_t s);
 cudaError_t launch_two2_f16(const Fused2Args<__half, float> &a, int rows, cudaStream_t s);
+constexpr int TWO_COLUMNS = 122; // of a strip, at most
 struct TwoUnit;
 cudaError_t launch_batch_two_f32(const Fused2Args<float, float> *doms, const TwoUnit *units, int nunits,
                                  int parity, int flags, cudaStream_t s);

@@ -30,12 +30,15 @@ inline bool flat_beats_tile(size_t nx, size_t ny, sclbm_precision p, bool solid)
 
 // Whether bands of a height of the caller's choice (0: none) run in pairs
 // (fused_two.cuh).  A band of r rows computes r + 4 rows of the first step, so low
-// ones lose to single steps of that height.  us per step, pairs / single steps:
-// FP32 2048^2 2 rows 151 / 121, 512^2 3 rows 11.2 / 10.4, 4 rows equal or faster; FP16
-// 2048^2 4 rows 115 / 103, 5 rows 104 / 100, 6 rows equal or faster.
-inline bool two_rows_pay(sclbm_precision p, int rows)
+// ones lose to single steps of that height, unless all units (four CTAs per SM)
+// are under way at once and latency counts.  us per step, pairs / single steps:
+// FP32 2048^2 2 rows 151 / 121, 512^2 3 rows 11.2 / 10.4, 1024^2 3 rows 33.7 / 37.1, 256^2
+// 2 rows 5.6 / 6.3; FP16 2048^2 4 rows 115 / 103, 5 rows 104 / 100, 6 rows equal or
+// faster, 300^2 5 rows 7.0 / 10.4, with solid nodes 1024^2 3 rows 42.3 / 39.1, 4 rows
+// equal, 5 rows 35.7 / 41.0.
+inline bool two_rows_pay(sclbm_precision p, int rows, long units, bool solid, int sms)
 {
-    return rows == 0 || rows >= (p == SCLBM_FP32_SHIFTED ? 4 : 6);
+    return rows == 0 || units <= 4L * sms || rows >= (p == SCLBM_FP32_SHIFTED ? 3 : solid ? 4 : 6);
 }
 
 // Whether an FP16 batch with solid nodes, off the ring body, runs in pairs or in

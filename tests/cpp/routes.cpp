@@ -24,8 +24,8 @@ int main()
             std::cin >> nx >> ny >> p >> keep;
             std::cout << flat_beats_tile(nx, ny, (sclbm_precision)p, keep != 0) << '\n';
         } else if (what == "rows") { // bands of this height in pairs
-            std::cin >> p >> n;
-            std::cout << two_rows_pay((sclbm_precision)p, n) << '\n';
+            std::cin >> p >> n >> K >> keep >> sms; // height, units, solid nodes
+            std::cout << two_rows_pay((sclbm_precision)p, n, K, keep != 0, sms) << '\n';
         } else if (what == "warp") { // rows of strips, thousandths of their columns, SMs
             std::cin >> n >> K >> sms;
             std::cout << batch_two_beats_warp(n, K / 1000.0, sms) << '\n';

@@ -82,11 +82,13 @@ def test_single_steps_off_the_ring(ask):
 
 
 def test_low_bands_take_single_steps(ask):
-    """us per step, pairs / single steps: FP32 3 rows 11.2 / 10.4, 4 rows equal; FP16
-    5 rows 104 / 100, 6 rows equal."""
-    least = {FP32: 4, FP16: 6}
-    questions = [("rows", p, n) for p in least for n in (0, 1, 2, 3, 4, 5, 6, 7, 64)]
-    assert ask(questions) == [(int(n == 0 or n >= least[p]),) for _, p, n in questions]
+    """us per step, pairs / single steps: FP32 1024^2 3 rows 33.7 / 37.1, 2 rows 42 / 37,
+    256^2 2 rows (384 units) 5.6 / 6.3; FP16 2048^2 5 rows 104 / 100, with solid nodes 126 /
+    132, 1024^2 3 rows with solid nodes 42.3 / 39.1, 300^2 3 rows (300 units) 7.4 / 8.4."""
+    least = {(FP32, 0): 3, (FP32, 1): 3, (FP16, 0): 6, (FP16, 1): 4}
+    questions = [("rows", p, n, 3000, solid, SMS) for p, solid in least for n in (0, 1, 2, 3, 4, 5, 6, 7, 64)]
+    assert ask(questions) == [(int(n == 0 or n >= least[p, solid]),) for _, p, n, _, solid, _ in questions]
+    assert ask([("rows", FP32, 2, 384, 0, SMS), ("rows", FP16, 3, 300, 0, SMS)]) == [(1,), (1,)]
 
 
 def test_narrow_fp16_domains_with_solid_nodes(ask):
