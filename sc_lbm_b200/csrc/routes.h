@@ -58,12 +58,14 @@ inline bool batch_two_beats_warp(double rows, double full, int sms) { return row
 // per thread / ring: 2 x 1024^2 with disks of radius 10-30 (0.027) 139 / 155, 4-16
 // (0.052) 155 / 163, 2-4 (0.079) 179 / 173, 10 % of all nodes solid (0.18) 198 / 183;
 // 24 x (400 x 306), strips 78 % full, (0.027) 203 / 257, (0.18) 272 / 285; 16 x 512^2
-// (0.056) 309 / 301; 200 x (320 x 160) 769 / 784; 4 x 256^2 (0.18) 20 / 28.
+// (0.056) 309 / 301; 200 x (320 x 160) 769 / 784; 4 x 256^2 (0.18) 20 / 28; every fourth
+// node solid (0.375), 4 x 512^2 100 / 107, 256 x 64^2, strips half full, 97 / 143, 24 x
+// (400 x 306) 280 / 288, 64 x (300 x 200) 401 / 371.
 inline bool batch_flat_beats_ring(double nodes, double full, double changes)
 {
-    if (nodes < 1e6) return true;
+    if (nodes < 1.2e6 || (nodes < 8e6 && full < 0.7)) return true;
     const bool loose = full < 0.9;
-    if (nodes < 4e6) return changes < (loose ? 0.15 : 0.06);
+    if (nodes < 4e6) return changes < (!loose ? 0.06 : nodes < 3e6 ? 0.5 : 0.15);
     return nodes < 8e6 && loose && changes < 0.06;
 }
 

@@ -104,6 +104,8 @@ def test_narrow_fp16_domains_with_solid_nodes(ask):
 BATCH64 = [
     ((262, 1000, 180), True),                             # 4 x 256^2 20 / 28
     ((979, 781, 180), True),                              # 8 x (400 x 306) 94 / 100
+    ((1049, 500, 375), True), ((1049, 1000, 375), True),  # 256 x 64^2 97 / 143; 4 x 512^2 100 / 107
+    ((2938, 781, 375), True), ((3840, 781, 375), False),  # 24 x (400 x 306) 280 / 288; 64 x (300 x 200) 401 / 371
     ((1311, 1000, 56), True), ((1311, 1000, 95), False),  # 5 x 512^2 100 / 106; 115 / 113
     ((2097, 1000, 52), True), ((2097, 1000, 79), False),  # 2 x 1024^2 155 / 163; 179 / 173
     ((2938, 781, 118), True),                             # 24 x (400 x 306) 255 / 276
