@@ -262,22 +262,30 @@ int sclbm_domain_download_mask(sclbm_domain *d, int32_t *mask, size_t count);
 int sclbm_domain_download_rho(sclbm_domain *d, int comp, double *rho, size_t count);
 int sclbm_domain_download_velocity(sclbm_domain *d, int comp, double *ux, double *uy,
                                    size_t count);
-/* advance nsteps time steps (queued on the library stream, not synchronised) */
+/* advance nsteps time steps (queued on the library stream, not synchronised).
+ * A call may be captured into a CUDA graph; the graph holds the addresses of the
+ * domain's buffers.  From then on every call leaves the state where as many
+ * single steps would: capture an even number of steps to replay it at will, also
+ * between calls made outside it that take an even number. */
 int sclbm_domain_step(sclbm_domain *d, int nsteps);
 /* Per component: total mass, x and y momentum over fluid nodes, reduced in
  * FP64 (out[3*comp + 0..2]); out[6] = number of non-finite populations. */
 int sclbm_domain_mass_momentum(sclbm_domain *d, double out[7]);
 /* Kernel selection (all variants give identical results):
  *   0 = automatic (default): the fastest measured form -- one component:
- *       several steps per launch; two components: two steps per launch for
- *       FP32 beyond 450 k and FP16 beyond 1.5 M nodes, one node per thread
- *       below and for FP64 up to 4 M nodes, the ring kernel (rows on 16-byte
- *       boundaries; FP64: the depth of 12 and 16-row bands; FP32: the depth
- *       of 13 and 24-row bands; FP16: the depth of 12 and 32-row bands) for
- *       larger FP64 lattices and an odd last step.  With tile_y or threads of
- *       the caller's choice: two steps per launch in bands of tile_y rows
- *       (FP32, FP16), else the ring where its bands fill three waves of the
- *       GPU, else 8 for FP32/FP16 storage with solid nodes, 2 otherwise;
+ *       several steps per launch (lattices a few nodes wide, and one step a
+ *       call on large ones: one node per thread); two components: two steps
+ *       per launch for FP32 beyond 450 k and FP16 beyond 1.5 M nodes; single
+ *       steps (smaller lattices, FP64, an odd last step): the ring kernel (rows
+ *       on 16-byte boundaries; FP64: the depth of 12 and 16-row bands; FP32:
+ *       the depth of 13 and 24-row bands; FP16: the depth of 12 and 32-row
+ *       bands) where its bands fill three waves of the GPU and, for FP64, from
+ *       4 M nodes; else one node per thread; on large FP32/FP16 lattices off
+ *       16-byte rows 2 or 8.  With a tile_y of the caller's choice: two steps
+ *       per launch in bands of tile_y rows (FP32 from three rows, FP16 from six,
+ *       with solid nodes four; lower ones on small lattices); else, and with
+ *       threads of the caller's choice, the ring where its bands fill three
+ *       waves, else 8 for FP32/FP16 storage with solid nodes, 2 otherwise;
  *   1 = two pass (density kernel, then the fused kernel reading it);
  *   2 = single pass, one tile per CTA, population rows held in registers;
  *   3 = single pass, population rows staged through a shared-memory ring by
@@ -452,20 +460,26 @@ int sclbm_domain_halo_min_unpack(sclbm_domain *d, int side, const void *src);
 int sclbm_domain_step_rows(sclbm_domain *d, int row0, int nrows, int finish);
 
 /* ------------------------------------------------------------------- batch
- * Many independent domains of one precision advanced together: one launch
- * per time step walks a tile list drawn from all domains, and the launch
+ * Many independent domains of one precision advanced together by one launch
+ * per time step or per two, over tiles drawn from all domains; the launch
  * sequence of a run is captured in a CUDA graph. */
 typedef struct sclbm_batch sclbm_batch;
 
-/* tile_y_per_domain may be NULL: rows per tile then come from the tuned table
- * (sclbm_tuned_config) for each domain's size class */
+/* tile_y_per_domain may be NULL, the best choice unless another was measured:
+ * the one-step bodies' rows per tile then come from the tuned table
+ * (sclbm_tuned_config) for each domain's size class, those of pairs from the
+ * sizes of the whole batch.  Heights given are rows per tile, unit or band of
+ * whichever body runs; they keep FP64 batches off one node per thread, and
+ * FP32/FP16 ones below the heights that domain variant 0 takes in pairs. */
 int sclbm_batch_create(sclbm_domain *const *domains, int ndomains, const int *tile_y_per_domain,
                        sclbm_batch **out);
 void sclbm_batch_destroy(sclbm_batch *b);
 /* Work decomposition (same results either way): 0 = automatic (FP32, FP16: two
- * steps per launch, a CTA per strip and band; FP64 with solid nodes or fewer
- * than 4 M nodes in all and no tile_y_per_domain: one node per thread; else,
- * and for steps left over, batches with solid nodes: the body the autotuner's mixed-ensemble sweep found fastest
+ * steps per launch, a CTA per strip and band, but for FP16 batches of many narrow
+ * domains with solid nodes; FP64 without tile_y_per_domain: one node per thread
+ * below 4 M nodes in all and, with solid nodes, where it beats the ring by size,
+ * widths and how scattered they are; else, and for steps left over, batches with
+ * solid nodes: the body the autotuner's mixed-ensemble sweep found fastest
  * for the precision -- the ring body 11 with 16-row units for FP64, 24 for
  * FP32 and 32 for FP16; other batches: the tuned variant of the size
  * class holding most of the batch's nodes); 11 = ring body: persistent CTAs
@@ -488,9 +502,11 @@ int sclbm_batch_set_kernel(sclbm_batch *b, int variant);
 int sclbm_batch_step(sclbm_batch *b, int nsteps, int use_graph);
 int sclbm_batch_info(const sclbm_batch *b, int *ntiles, int *grid_ctas);
 
-/* Tuned launch shape for an nx x ny two-component domain stored at
+/* Tuned launch shape of the one-step batch bodies (2: tile list of tile_y rows,
+ * 3: strips x bands) for an nx x ny two-component domain stored at
  * `precision` (sclbm_precision; -1 = the recommended one), from the table
- * that sc_lbm_b200/autotune.py measured on B200 and the build compiled in.
+ * that sc_lbm_b200/autotune.py measured on B200 and the build compiled in; the
+ * default bodies (pairs, one node per thread) are not in it and are faster.
  * Sizes outside the table take the nearest size class.  *recommended is the
  * fastest storage whose density error against FP64 stayed within 1e-5 for
  * that class.  Host-only lookup (no device needed).  No reference

@@ -397,7 +397,7 @@ class Domain(_Handle):
 
 
 class Batch(_Handle):
-    """Many domains advanced together by one launch per step (CUDA graph)."""
+    """Many domains advanced together, one launch per step or per two steps (CUDA graph)."""
     _destroy = "sclbm_batch_destroy"
 
     def __init__(self, domains, tile_y=None):
@@ -420,8 +420,10 @@ class Batch(_Handle):
 
 
 def tuned_config(nx: int, ny: int, precision: int | None = None) -> dict:
-    """Tuned batch launch shape for an nx x ny domain (host lookup in the
-    autotuned table): {"tile_y", "variant", "recommended_precision"}."""
+    """Tuned shape of the one-step batch bodies for an nx x ny domain (host lookup
+    in the autotuned table): {"tile_y", "variant", "recommended_precision"}.  A
+    batch uses it by itself where it needs it; leave tile_y and the variant at
+    their defaults, which also allow pairs and one node per thread."""
     t, v, r = C.c_int(), C.c_int(), C.c_int()
     call("sclbm_tuned_config", int(nx), int(ny), -1 if precision is None else int(precision),
          C.byref(t), C.byref(v), C.byref(r))

@@ -5,7 +5,9 @@
 For every domain size class of the ensemble workload (Nx in 64..512, Ny in
 64..256) it builds a batch of seeded porous domains of the class's
 representative size and times one persistent launch per step (CUDA graph)
-over the candidate shapes of each storage precision:
+over the candidate shapes of each storage precision (the one-step bodies, asked
+for by name; pairs and one node per thread, which batches take by default, have
+no shape to tune here):
 
 * tile list (variant 2) with tile_y = 4, 8, 16, 32, 64 rows per tile -- the
   nodes each thread advances per tile (one column per thread, 128 threads);
@@ -23,7 +25,7 @@ ring bodies (variants 11 and 12: 128- and 64-column strips) at several rows
 per unit, the tile lists (2 register tile, 8 uniform solid form, 9 half
 tiles, 10 one-warp tiles) at several rows per tile, and the strips x bands
 body (3) -- per storage precision.  The fastest becomes the `batch_default`
-of that precision, the body every batch with solid nodes starts with.  The
+of that precision, the one-step body of batches with solid nodes.  The
 JSON it writes is compiled into the library by build.py (sclbm_tuned_config,
 the size-class tile heights and the batch defaults).
 """

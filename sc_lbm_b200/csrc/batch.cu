@@ -1,18 +1,31 @@
 // batch.cu -- many independent two-component domains advanced together, one
-// persistent launch per time step, the launches of a run captured once into a
+// launch per step or per two steps, the launches of a run captured once into a
 // CUDA graph and replayed.  All domains of a batch share the storage precision
-// and the buffer parity.  Two work decompositions:
+// and the buffer parity.  The bodies that variant 0 takes:
 //
-//  * bands (FP64/FP32): every domain is cut into 128-column strips and row
-//    bands of one common height, chosen as the smallest for which all
-//    (domain, strip, band) tiles are resident at once; neighbouring strips of
-//    a band are adjacent in the list so they walk the same rows together; the
-//    pipelined single-pass body (fused_async.cuh) runs each tile;
-//  * tile list: every tile (126 columns x tile_y rows) of every domain,
-//    largest first; CTA b takes tiles b, b+grid, ... and runs the
-//    register-tile body (batch_kernel.cuh).
-// The automatic choice and the rows per tile come from the autotuned size-class
-// table (tuning.h), weighted by the nodes of each class in the batch.
+//  * pairs (FP32/FP16, k_batch_two in fused_two.cuh): every domain is cut into
+//    strips of up to 122 columns and bands of rows, a CTA per strip and band, two
+//    steps per launch;
+//  * one node per thread (FP64, k_batch_flat in fused_flat.cuh): a CTA per tile of
+//    32 x 4 nodes, on all-fluid batches below 4 M nodes and, with solid nodes, where
+//    it beats the ring (routes.h);
+//  * for what these leave (steps left over from pairs, lattices or heights that
+//    pairs do not take, larger FP64 batches) and by set_kernel the persistent
+//    one-step bodies:
+//    - ring (fused_ring.cuh): CTAs take units of a strip and a band from a
+//      counter; the automatic choice with solid nodes on rows that start on
+//      16-byte boundaries;
+//    - bands (FP64/FP32): every domain is cut into 128-column strips and row
+//      bands of one common height, chosen as the smallest for which all
+//      (domain, strip, band) tiles are resident at once; neighbouring strips of
+//      a band are adjacent in the list so they walk the same rows together; the
+//      pipelined single-pass body (fused_async.cuh) runs each tile;
+//    - tile list: every tile (126 columns x tile_y rows) of every domain,
+//      largest first; CTA b takes tiles b, b+grid, ... and runs the
+//      register-tile body (batch_kernel.cuh).
+// Among the persistent bodies the automatic choice and the rows per tile come
+// from the autotuned size-class table (tuning.h), weighted by the nodes of each
+// class in the batch.
 #include <algorithm>
 #include <memory>
 #include <numeric>

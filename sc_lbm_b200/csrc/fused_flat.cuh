@@ -6,7 +6,9 @@
 // step, 8 % of the warps busy).  Here every node has a thread, so one load
 // round, one barrier and one collision are all there is; what bounds it is that
 // chain's latency on small lattices, then L2 (512^2 FP64: 374 B per node
-// counting the halo, 8 TB/s), and DRAM once both buffers outgrow L2.
+// counting the halo, 8 TB/s), and DRAM once both buffers outgrow L2; FP64 runs into
+// the board's power limit within a third of a second (1.49 of 1.965 GHz at 995 W:
+// 1024^2 54 -> 61 us).
 //
 // A CTA owns a tile of 32 columns and four rows, a warp per row (eight rows
 // have fewer halo nodes but ran 5-15 % slower above 256^2).  Each thread loads

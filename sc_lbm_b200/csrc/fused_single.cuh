@@ -10,6 +10,8 @@
 // Measured on one B200, us per step, one step per launch before and K steps now
 // (K by single_depth): FP64 200 x 50 4.7 -> 1.2, 700 x 333 8.2 -> 5.3, 4096^2 439
 // -> 306; FP32 200 x 50 4.15 -> 0.85, 1024^2 18.6 -> 13.0, 4096^2 273 -> 196.
+// Lattices a few nodes wide, and large ones stepped one step a call, do not fill
+// the tiles or pay for the halo in vain: they take one node per thread (routes.h).
 // Small lattices are bound by the chain of a step (loads from shared memory, a
 // collision, a barrier) and a launch every K steps, large ones by instructions:
 // the halo's repeated work against the DRAM traffic it saves.

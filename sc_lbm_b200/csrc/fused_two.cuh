@@ -4,9 +4,12 @@
 // Why.  A step on its own reads and writes every population once, and the
 // one-step kernels run at the memory's copy rate on large lattices.  Two steps
 // per pass read and write the populations once for both: the state between the
-// steps lives in shared memory, a few rows at a time.  What bounds it then is
-// the FP32 pipe (packed instructions: 58 % busy) and, over seconds, the
-// board's power limit; DRAM is half busy.  Measured on one B200, us per step
+// steps lives in shared memory, a few rows at a time.  Nothing is saturated then:
+// issue slots 55-64 % taken, the FP32 pipe about 56 % busy (a packed pair takes two
+// cycles), DRAM 24-45 %.  Three warps per scheduler share 316-410 instructions per
+// node and step, and the largest stall is their fixed latency.  FP32 also runs into
+// the board's power limit within half a second (1.65 of 1.965 GHz at 995 W: 267 ->
+// 291 us on 4096^2); FP16 does not.  Measured on one B200, us per step
 // (the one-step kernels before): FP32 4096^2 267 (407), its 60 % fluid form 322
 // (459), FP16 4096^2 277 (334) and 324 (442), FP32 2048 x 1024 with 40 % solid
 // nodes 46 (78), 1024^2 22.6 (35.5).  With solid nodes a node step took 469

@@ -1,12 +1,13 @@
 // launch.cuh -- kernels launched as programmatic dependents of the one before.
 //
 // A kernel launched this way may start while the kernel before it in the
-// stream drains, which hides its launch latency; it calls dependent_wait
-// before it touches memory, and dependent_launch after that, so at most two
-// kernels of a chain are under way and the one before them has ended: with two
-// buffers in turn, nothing that a kernel writes is still being read.  Data of
-// the kernel before is read with ordinary loads (the read-only path may hold
-// lines from before the wait).
+// stream drains, which hides its launch latency.  Before dependent_wait it reads
+// only what no kernel in the stream writes (a batch's tile list and argument
+// blocks, which a copy waited for brought there), and writes nothing outside its
+// CTA; dependent_launch follows the wait, so at most two kernels of a chain are
+// under way and the one before them has ended: with two buffers in turn, nothing
+// that a kernel writes is still being read.  Data of the kernel before is read
+// with ordinary loads (the read-only path may hold lines from before the wait).
 #pragma once
 #include <cuda_runtime.h>
 

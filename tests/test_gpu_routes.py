@@ -144,3 +144,28 @@ def test_fp64_batch_of_scattered_solids(sclbm, radii, flat):
         one.init_noise(c, 1.0, 0.1, 3 + c)
     one.step(3)
     assert all(d.download_f(0).tobytes() == one.download_f(0).tobytes() for d in doms)
+
+
+@pytest.mark.parametrize("prec_name,rows", [("FP32_SHIFTED", 16), ("FP16_SHIFTED", 16), ("FP16_SHIFTED", 0)])
+def test_disks_added_on_the_device_reach_the_node_codes(sclbm, prec_name, rows):
+    """Pairs and the FP16 form of one node per thread read node codes, the register
+    tile the mask: the same bytes after disks are added, and as on a domain made
+    from the finished mask."""
+    nx, ny = 150, 131
+    p = sclbm.make_params(g_fluid=(0.9, 0.9), g_solid=(-0.1, 0.1))
+    disks = dict(porosity=0.7, rmin=3, rmax=9, seed=11)
+    out = []
+    for variant, r in ((0, rows), (2, 0), (0, rows)):
+        mask = np.ones(nx * ny, np.int32)
+        if len(out) == 2:
+            mask = packed
+        d = sclbm.Domain(nx, ny, mask, p, getattr(sclbm, prec_name))
+        if len(out) < 2:
+            assert d.add_random_disks(**disks) > 0
+            packed = d.download_mask()
+        d.set_kernel(variant, r)
+        for k in range(2):
+            d.init_noise(k, 1.0, 0.1, 3 + k)
+        d.step(5)
+        out.append([d.download_f(k).tobytes() for k in range(2)])
+    assert out[0] == out[1] == out[2]
