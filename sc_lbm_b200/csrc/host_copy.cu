@@ -16,7 +16,7 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <system_error>
+#include <exception>
 #include <thread>
 
 #include "internal.h"
@@ -70,7 +70,7 @@ void host_pages_in(void *dst, size_t bytes)
     int k = 1;
     try {
         for (; k < n; ++k) helpers[k] = std::thread(part, k);
-    } catch (const std::system_error &) { // no more threads: the copy takes these faults
+    } catch (const std::exception &) { // no more threads: the copy takes these faults
     }
     part(0);
     for (int j = 1; j < k; ++j) helpers[j].join();
