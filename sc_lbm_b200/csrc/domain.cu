@@ -524,7 +524,8 @@ static int domain_launch_two(sclbm_domain *d, cudaStream_t s)
 cudaStream_t domain_stream(sclbm_domain *d)
 {
     cudaStream_t s = stream();
-    if (!d->held) d->held = being_captured(s);
+    // two FP64 components take one step per launch: their buffers keep their names
+    if (!d->held && (d->ncomp == 1 || d->prec != SCLBM_FP64)) d->held = being_captured(s);
     return s;
 }
 
